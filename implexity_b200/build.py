@@ -23,7 +23,15 @@ MMA_SOURCE = CSRC / "mma_cpu.cpp"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
-SOURCES = ["lbm_forward.cu", "lbm_adjoint.cu", "lbm_misc.cu", "lbm_noalloc.cu", "lbm_runtime.cpp"]
+SOURCES = ["lbm_forward.cu", "lbm_adjoint.cu", "lbm_march.cu", "lbm_misc.cu", "lbm_noalloc.cu", "lbm_runtime.cpp"]
+# The stepping kernels' instances compile as one unit per lattice and collision
+# (LBM_PART: 10 * lattice + CollKind), in parallel with the rest.  (nvcc's own
+# --split-compile makes them spill: 0 -> 108 bytes in the FP32 forward step,
+# which then takes 149 instead of 124 us at 256x128x128.)
+PARTS = {"lbm_forward.cu": [190, 191, 192, 270, 271, 272], "lbm_adjoint.cu": [190, 191, 192, 270, 271, 272],
+         "lbm_march.cu": [190, 192, 270, 272]}
+UNITS = [(src, part) for part in (191, 271, 190, 270, 192, 272, None) for src in SOURCES
+         if part is None or part in PARTS.get(src, ())]
 
 
 def nvcc() -> str:
@@ -78,19 +86,21 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
     headers = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + sorted(INCLUDE.glob("*.h"))
 
-    def compile_one(src: str) -> Path:
-        obj = BUILD / (src + ".o")
+    def compile_one(unit: tuple[str, int | None]) -> Path:
+        src, part = unit
+        obj = BUILD / (src + (".o" if part is None else f".{part}.o"))
         deps = [CSRC / src, *headers]
         if not force and obj.exists() and all(d.stat().st_mtime <= obj.stat().st_mtime for d in deps):
             return obj
-        cmd = [cc, *ARCH, *FLAGS, "-c", str(CSRC / src), "-o", str(obj)]
+        define = [] if part is None else [f"-DLBM_PART={part}"]
+        cmd = [cc, *ARCH, *FLAGS, *define, "-c", str(CSRC / src), "-o", str(obj)]
         if verbose:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
         return obj
 
-    with ThreadPoolExecutor(max_workers=len(SOURCES)) as ex:
-        objs = list(ex.map(compile_one, SOURCES))
+    with ThreadPoolExecutor(max_workers=max(2, os.cpu_count() or 2)) as ex:
+        objs = list(ex.map(compile_one, UNITS))
     tmp = LIB.with_suffix(".so.tmp")
     cmd = [cc, *ARCH, "-shared", "-o", str(tmp), *map(str, objs)]
     if verbose:

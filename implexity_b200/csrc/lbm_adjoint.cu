@@ -12,7 +12,17 @@
 // forward step (lbm_device.cuh).
 #include "lbm_device.cuh"
 
+// Compiled once per lattice and collision (LBM_PART) for the kernels, and once
+// without it for the entry point.
 namespace lbm {
+cudaError_t adjoint_190(int storage, const AdjArgs& a, cudaStream_t s);
+cudaError_t adjoint_191(int storage, const AdjArgs& a, cudaStream_t s);
+cudaError_t adjoint_192(int storage, const AdjArgs& a, cudaStream_t s);
+cudaError_t adjoint_270(int storage, const AdjArgs& a, cudaStream_t s);
+cudaError_t adjoint_271(int storage, const AdjArgs& a, cudaStream_t s);
+cudaError_t adjoint_272(int storage, const AdjArgs& a, cudaStream_t s);
+
+#ifdef LBM_PART
 namespace {
 
 template <int Q, typename T, int NREC>
@@ -219,6 +229,11 @@ cudaError_t run_adjoint(const AdjArgs& a, cudaStream_t s) {
 
 }  // namespace
 
+cudaError_t LBM_PART_NAME(adjoint)(int storage, const AdjArgs& a, cudaStream_t s) {
+    LBM_STORAGE_DISPATCH(storage, T, return run_adjoint<LBM_PART / 10, LBM_PART % 10, T>(a, s))
+    return cudaErrorInvalidValue;
+}
+#else
 cudaError_t launch_adjoint(int Q, int coll, int lstorage, const AdjArgs& a0, int grid, cudaStream_t s) {
     (void)grid;
     AdjArgs a = a0;
@@ -234,24 +249,10 @@ cudaError_t launch_adjoint(int Q, int coll, int lstorage, const AdjArgs& a0, int
         !staged_aligned(a.record, a.rec0, a.rec_planes, 4) ||
         !staged_aligned(a.mask, nullptr, 0, 4) || !staged_aligned(a.alpha, nullptr, 0, 4))
         return cudaErrorMisalignedAddress;
-    if (Q == 19) {
-        if (coll == CK_MRT) {
-            LBM_STORAGE_DISPATCH(lstorage, T, return run_adjoint<19, CK_MRT, T>(a, s))
-        } else if (coll == CK_MRT_BULK) {
-            LBM_STORAGE_DISPATCH(lstorage, T, return run_adjoint<19, CK_MRT_BULK, T>(a, s))
-        } else {
-            LBM_STORAGE_DISPATCH(lstorage, T, return run_adjoint<19, CK_PAIRS, T>(a, s))
-        }
-    } else {
-        if (coll == CK_MRT) {
-            LBM_STORAGE_DISPATCH(lstorage, T, return run_adjoint<27, CK_MRT, T>(a, s))
-        } else if (coll == CK_MRT_BULK) {
-            LBM_STORAGE_DISPATCH(lstorage, T, return run_adjoint<27, CK_MRT_BULK, T>(a, s))
-        } else {
-            LBM_STORAGE_DISPATCH(lstorage, T, return run_adjoint<27, CK_PAIRS, T>(a, s))
-        }
-    }
-    return cudaGetLastError();
+    if (Q == 19)
+        return coll == CK_MRT ? adjoint_191(lstorage, a, s) : coll == CK_MRT_BULK ? adjoint_192(lstorage, a, s) : adjoint_190(lstorage, a, s);
+    return coll == CK_MRT ? adjoint_271(lstorage, a, s) : coll == CK_MRT_BULK ? adjoint_272(lstorage, a, s) : adjoint_270(lstorage, a, s);
 }
+#endif
 
 }  // namespace lbm

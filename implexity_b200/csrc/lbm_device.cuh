@@ -1416,6 +1416,11 @@ __device__ void finish_sums(Sums<NS> v, double* out, const Reduce& red) {
 
 
 // ------------------------------------------------------------------ launch helpers
+// name_<LBM_PART>: the kernels' units are compiled per lattice and collision.
+#define LBM_PASTE_(a, b) a##_##b
+#define LBM_PASTE(a, b) LBM_PASTE_(a, b)
+#define LBM_PART_NAME(name) LBM_PASTE(name, LBM_PART)
+
 #define LBM_STORAGE_DISPATCH(storage, T, ...)            \
     switch (storage) {                                   \
         case ST_F32: {                                   \

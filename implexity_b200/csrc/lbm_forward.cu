@@ -13,7 +13,17 @@
 // system sustains about a third more bandwidth than the in-place AA pattern.
 #include "lbm_device.cuh"
 
+// Compiled once per lattice and collision (LBM_PART) for the kernels, and once
+// without it for the entry point.
 namespace lbm {
+cudaError_t forward_190(int storage, const FwdArgs& a, cudaStream_t s);
+cudaError_t forward_191(int storage, const FwdArgs& a, cudaStream_t s);
+cudaError_t forward_192(int storage, const FwdArgs& a, cudaStream_t s);
+cudaError_t forward_270(int storage, const FwdArgs& a, cudaStream_t s);
+cudaError_t forward_271(int storage, const FwdArgs& a, cudaStream_t s);
+cudaError_t forward_272(int storage, const FwdArgs& a, cudaStream_t s);
+
+#ifdef LBM_PART
 namespace {
 
 template <int Q, typename T>
@@ -271,6 +281,11 @@ cudaError_t run_forward(const FwdArgs& a, cudaStream_t s) {
 
 }  // namespace
 
+cudaError_t LBM_PART_NAME(forward)(int storage, const FwdArgs& a, cudaStream_t s) {
+    LBM_STORAGE_DISPATCH(storage, T, return run_forward<LBM_PART / 10, LBM_PART % 10, T>(a, s))
+    return cudaErrorInvalidValue;
+}
+#else
 bool staged_aligned(const void* base, const int64_t* run0, int nrun, size_t elem) {
     const uintptr_t b = reinterpret_cast<uintptr_t>(base);
     if (b % 16) return false;
@@ -301,24 +316,10 @@ cudaError_t launch_forward(int Q, int coll, int storage, const FwdArgs& a0, int 
     if (!staged_aligned(a.src, a.run0, Q, es) || !staged_aligned(a.mask, nullptr, 0, 4) ||
         !staged_aligned(a.alpha, nullptr, 0, 4) || (a.bulk_store && !staged_aligned(a.dst, nullptr, 0, es)))
         return cudaErrorMisalignedAddress;
-    if (Q == 19) {
-        if (coll == CK_MRT) {
-            LBM_STORAGE_DISPATCH(storage, T, return run_forward<19, CK_MRT, T>(a, s))
-        } else if (coll == CK_MRT_BULK) {
-            LBM_STORAGE_DISPATCH(storage, T, return run_forward<19, CK_MRT_BULK, T>(a, s))
-        } else {
-            LBM_STORAGE_DISPATCH(storage, T, return run_forward<19, CK_PAIRS, T>(a, s))
-        }
-    } else {
-        if (coll == CK_MRT) {
-            LBM_STORAGE_DISPATCH(storage, T, return run_forward<27, CK_MRT, T>(a, s))
-        } else if (coll == CK_MRT_BULK) {
-            LBM_STORAGE_DISPATCH(storage, T, return run_forward<27, CK_MRT_BULK, T>(a, s))
-        } else {
-            LBM_STORAGE_DISPATCH(storage, T, return run_forward<27, CK_PAIRS, T>(a, s))
-        }
-    }
-    return cudaGetLastError();
+    if (Q == 19)
+        return coll == CK_MRT ? forward_191(storage, a, s) : coll == CK_MRT_BULK ? forward_192(storage, a, s) : forward_190(storage, a, s);
+    return coll == CK_MRT ? forward_271(storage, a, s) : coll == CK_MRT_BULK ? forward_272(storage, a, s) : forward_270(storage, a, s);
 }
+#endif
 
 }  // namespace lbm

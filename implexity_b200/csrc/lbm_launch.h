@@ -82,6 +82,45 @@ struct AdjArgs {
     const float* omega_cell; // per-cell relaxation rate 1/tau (BGK; nullptr: the uniform rate of P)
 };
 
+// One warp's share of a pass's admission record (k_march_forward).
+struct StepPartial {
+    double mass, exch;
+    float min_f, max_u2;
+    int32_t nonfinite, pad;
+};
+
+// A run of forward passes in one cooperative launch (lbm_march.cu): pass 0
+// reads a.src, the passes write a.dst and dst1 in turn.  a.record, diag and
+// a.stage (the response sums of every pass) point at the first pass's slot;
+// a.apply_ports holds for pass 0, the later ones apply every port.
+struct MarchFwdArgs {
+    FwdArgs a;
+    void* dst1;
+    int32_t n_pass;
+    int32_t inspect_last;   // the last pass loads only
+    int32_t n_ports;        // port maps of one pass
+    int32_t port_stride;    // maps from one pass to the next (0: the same)
+    int64_t record_stride;  // floats from one pass's record to the next
+    StepDiag* diag;         // one per pass (nullptr: off)
+    void* scratch;          // march_scratch() bytes per pass when diag or a.stage is set
+    int64_t scratch_bytes;
+    StepPartial* partial;   // set by the launcher
+    double* rpartial;
+    unsigned* bar;          // barrier counter
+};
+
+// A run of transposed steps: pass i reads record a.record - i * record_stride
+// and the maps a.ports - i * port_stride, a.src and a.dst swap every pass;
+// pass 0 reads with a.in_scale_inv, the later ones the scale they wrote.
+struct MarchAdjArgs {
+    AdjArgs a;
+    int32_t n_pass;
+    int32_t stage_passes;   // passes that add the response VJP of their state
+    int32_t n_ports, port_stride;
+    int64_t record_stride;
+    unsigned* bar;
+};
+
 struct ObjArgs {
     Geometry G;
     Physics P;
@@ -148,6 +187,10 @@ cudaError_t launch_init(int Q, int storage, const Geometry& G, const Physics& P,
                         int64_t c_begin, int64_t c_end, cudaStream_t s);  // cells [c_begin, c_end)
 cudaError_t launch_forward(int Q, int coll, int storage, const FwdArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_adjoint(int Q, int coll, int lstorage, const AdjArgs& a, int grid, cudaStream_t s);
+// Bytes of MarchFwdArgs::scratch one pass of a grid of n cells needs.
+int64_t march_scratch(int64_t n, int sms, bool stage);
+cudaError_t launch_march_forward(int Q, int coll, int storage, const MarchFwdArgs& g, cudaStream_t s);
+cudaError_t launch_march_adjoint(int Q, int coll, int lstorage, const MarchAdjArgs& g, cudaStream_t s);
 cudaError_t launch_wait_probe(int* err, uint64_t limit_ns, unsigned long long* waited_ns, cudaStream_t s);
 cudaError_t launch_objective(int Q, int storage, int lstorage, int mode, const ObjArgs& a, int grid,
                              cudaStream_t s);  // mode 0: responses/fields, 1: seed

@@ -391,12 +391,14 @@ struct lbm_handle {
     float beta = 0, eta = 0.5f, proj_a = 0, proj_den = 1;
     // --- device
     int device = 0, sms = 148;
+    bool cooperative = false;  // the device takes cooperative launches
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int64_t device_bytes = 0;
     DevBuf pop, mask, alpha, phi, raw, den, slope, cls_d, fixed_d, offsets_d, ports_d, partial, counter, diag;
     DevBuf lam, record, abar, abar_final, phibar, scale, grad, norm2, sums, scratch, errflag;
     DevBuf omega_cell, tau_state, tau_bar;
+    DevBuf march;  // partial records of the passes of one launch, and its barrier counter
     AdjState* slab_adj = nullptr;  // x-slab steady adjoint in progress (lbm_slab_adjoint_begin)
     int lam_storage = LBM_STORE_F32;
     // --- ports: normalised specs with their signals; pulsatile ports keep one
@@ -903,6 +905,9 @@ void validate_and_build(lbm_handle& h, const lbm_problem_t& p) {
     // --- device
     CK(cudaGetDevice(&h.device));
     CK(cudaDeviceGetAttribute(&h.sms, cudaDevAttrMultiProcessorCount, h.device));
+    int coop = 0;
+    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h.device));
+    h.cooperative = coop != 0;
     CK(cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking));
     CK(cudaEventCreate(&h.ev0));
     CK(cudaEventCreate(&h.ev1));
@@ -1017,6 +1022,84 @@ void inspect(lbm_handle& h, StepDiag* diag, float* record, bool record_s = false
     CK(launch_forward(h.Q, coll_kernel(h), h.storage, a, grid_for(h), h.stream));
 }
 
+// A run of passes in one cooperative launch (lbm_march.cu) where the grid is
+// small enough for it to win and nothing runs between two steps: not for
+// extrapolating ports (a second kernel moves their cotangents after every
+// step), the general MRT collision or x-slabs (halos).
+// The limits, us per step of the staged kernels / of a run (B200):
+//   cells                  27 648      262 144      614 400     1 032 192    2 097 152
+//   forward FP32       12.4 / 3.5  18.5 / 11.2  27.8 / 23.5  43.3 / 41.3  67.9 / 73.5
+//   forward FP16       14.4 / 3.5  19.5 / 11.1  25.5 / 18.7  37.1 / 32.1  62.5 / 60.2
+//   forward D3Q27      16.5 / 4.4  24.7 / 12.4  45.7 / 33.2  58.0 / 51.0   101 / 98
+//   forward FP64 coll. 16.2 / 4.8  27.0 / 15.3  44.8 / 34.9  71.9 / 55.6   116 / 107
+//   adjoint FP32        8.3 / 3.4  14.0 / 11.1  25.9 / 28.4  38.8 / 49.7
+//   adjoint FP16        8.3 / 3.3  12.5 / 10.7  20.6 / 18.6  32.8 / 37.2
+//   adjoint D3Q27      10.4 / 4.2  18.5 / 12.5  41.5 / 35.6  54.0 / 54.7
+// (FP64 collision at 4 194 304 cells: 224 / 216.)
+bool marches(const lbm_handle& h, bool adjoint) {
+    const int64_t most = adjoint ? (h.Q == 19 && h.lam_storage == LBM_STORE_F32 ? 400 << 10 : 640 << 10)
+                                 : (h.collision_fp64 ? 4 << 20 : 1 << 20);
+    return h.cooperative && h.n() <= most && coll_kernel(h) != CK_MRT && h.nee_groups.empty() && !h.slab;
+}
+
+// Passes of one launch: the partial records stay within 8 MB.
+int64_t march_chunk(lbm_handle& h, bool stage) {
+    const int64_t per = march_scratch(h.n(), h.sms, stage);
+    return std::max<int64_t>(8, std::min<int64_t>(128, (8 << 20) / per));
+}
+constexpr size_t MARCH_HEAD = 256;  // the barrier counter, ahead of the partial records
+
+// `passes` forward passes from the current state; with inspect_last the last
+// one is load-only (inspect), else every pass steps.  diag / record / stage
+// point at the first pass's slots (record_stride floats, 16 doubles apart).
+void run_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* diag, float* record, int64_t record_stride,
+                bool record_s, double* stage) {
+    if (passes < 3 || !marches(h, false)) {
+        for (int64_t i = 0; i < passes; ++i) {
+            StepDiag* d = diag ? diag + i : nullptr;
+            float* r = record ? record + (size_t)i * record_stride : nullptr;
+            double* st = stage ? stage + i * 16 : nullptr;
+            if (inspect_last && i == passes - 1) inspect(h, d, r, record_s, st);
+            else step(h, d, r, record_s, st);
+        }
+        return;
+    }
+    ensure_port_maps(h, h.t + passes);
+    const int64_t chunk = march_chunk(h, stage != nullptr);
+    const int64_t scratch = chunk * march_scratch(h.n(), h.sms, stage != nullptr);
+    h.march.alloc(MARCH_HEAD + (size_t)scratch, &h.device_bytes);
+    for (int64_t i = 0; i < passes;) {
+        const int64_t k = std::min(chunk, passes - i);
+        const bool inspects = inspect_last && i + k == passes;
+        MarchFwdArgs g{};
+        g.a = fwd_args(h);
+        g.a.apply_ports = h.pending ? 1 : 0;
+        g.a.record = record ? record + (size_t)i * record_stride : nullptr;
+        g.a.record_s = record_s ? 1 : 0;
+        g.a.stage = stage ? stage + i * 16 : nullptr;
+        g.a.step = (uint32_t)h.t;
+        g.dst1 = h.pop_array(h.cur) + pop_pad(h.G) * storage_bytes(h.storage);
+        g.n_pass = (int32_t)k;
+        g.inspect_last = inspects ? 1 : 0;
+        g.n_ports = h.n_ports;
+        g.port_stride = h.pulsatile ? h.n_ports : 0;
+        g.record_stride = record_stride;
+        g.diag = diag ? diag + i : nullptr;
+        g.bar = h.march.as<unsigned>();
+        g.scratch = h.march.as<char>() + MARCH_HEAD;
+        g.scratch_bytes = scratch;
+        CK(launch_march_forward(h.Q, coll_kernel(h), h.storage, g, h.stream));
+        const int64_t steps = k - (inspects ? 1 : 0);
+        if (steps > 0) {
+            h.cur ^= (int)(steps & 1);
+            h.restored = nullptr;
+            h.pending = h.n_ports > 0;
+            h.t += steps;
+        }
+        i += k;
+    }
+}
+
 void init_state(lbm_handle& h) {
     // both arrays: solid cells keep their populations in either
     const int64_t c0 = h.slab ? (int64_t)h.slab_hl * h.G.sx : 0;
@@ -1118,8 +1201,8 @@ lbm_status run_admitted(lbm_handle& h, int64_t steps, lbm_diag_t* out, int64_t K
     h.tavg_valid = false;
     if (averages) h.tsums.alloc((size_t)(steps + 1) * 16 * sizeof(double), ctr);
     CK(cudaEventRecord(h.ev0, h.stream));
-    for (int64_t s = 0; s < steps; ++s) {
-        if (K > 0 && s % K == 0) {
+    for (int64_t s = 0; s <= steps;) {
+        if (K > 0 && s < steps && s % K == 0) {
             // checkpoint of the state entering step s (scan.rs:181-196)
             Checkpoint c;
             c.buf = std::make_unique<DevBuf>();
@@ -1130,10 +1213,12 @@ lbm_status run_admitted(lbm_handle& h, int64_t steps, lbm_diag_t* out, int64_t K
             c.pending = h.pending;
             h.ckpts.push_back(std::move(c));
         }
-        double* slot = averages && s > 0 ? h.tsums.as<double>() + (size_t)s * 16 : nullptr;
-        step(h, d + s, nullptr, false, slot);
+        // up to the next checkpoint; the last run ends with the final inspection
+        const int64_t e = K > 0 && s / K * K + K < steps ? s / K * K + K : steps + 1;
+        run_passes(h, e - s, e == steps + 1, d + s, nullptr, 0, false,
+                   averages ? h.tsums.as<double>() + (size_t)s * 16 : nullptr);
+        s = e;
     }
-    inspect(h, d + steps, nullptr, false, averages ? h.tsums.as<double>() + (size_t)steps * 16 : nullptr);
     CK(cudaEventRecord(h.ev1, h.stream));
     std::vector<StepDiag>& hd = h.last_trajectory;
     hd.resize((size_t)steps + 1);
@@ -1307,6 +1392,48 @@ void adjoint_step(lbm_handle& h, AdjState& st, const float* rec, bool want_norm,
     ++st.steps;
 }
 
+// `count` transposed steps, the i-th linearised at record rec - i * stride and
+// state t - i (its port maps; state t throughout where stride is 0), with the
+// stage seed in the first stage_steps; the norm of the last one's result when
+// asked for.
+void adjoint_run(lbm_handle& h, AdjState& st, const float* rec, int64_t stride, int64_t count, bool want_norm, int64_t t,
+                 const SeedParams* stage = nullptr, int64_t stage_steps = 0, int rec_planes = 4) {
+    if (count < 2 || !marches(h, true)) {
+        for (int64_t i = 0; i < count; ++i)
+            adjoint_step(h, st, rec - i * stride, want_norm && i == count - 1, stride ? t - i : t,
+                         i < stage_steps ? stage : nullptr, rec_planes);
+        return;
+    }
+    h.march.alloc(MARCH_HEAD, &h.device_bytes);
+    for (int64_t i = 0; i < count;) {
+        const int64_t k = std::min<int64_t>(128, count - i);
+        MarchAdjArgs g{};
+        g.a = adj_args(h);
+        g.a.record = rec - i * stride;
+        g.a.rec_planes = rec_planes;
+        g.a.ports = ports_at(h, stride ? t - i : t);
+        if (stage) g.a.seed = *stage;
+        g.a.port_transpose = 1;
+        g.a.overwrite_abar = st.first ? 1 : 0;
+        g.a.in_scale_inv = 1.f / st.scale;
+        g.a.out_scale = st.target;
+        g.a.abar_factor = st.s0;
+        g.a.norm2 = want_norm && i + k == count ? h.norm2.as<double>() : nullptr;
+        g.n_pass = (int32_t)k;
+        g.stage_passes = (int32_t)std::max<int64_t>(0, std::min(k, stage_steps - i));
+        g.n_ports = h.n_ports;
+        g.port_stride = h.pulsatile && stride ? h.n_ports : 0;
+        g.record_stride = stride;
+        g.bar = h.march.as<unsigned>();
+        CK(launch_march_adjoint(h.Q, coll_kernel(h), h.lam_storage, g, h.stream));
+        h.lcur ^= (int)(k & 1);
+        st.scale = st.target;
+        st.first = false;
+        st.steps += k;
+        i += k;
+    }
+}
+
 double read_norm(lbm_handle& h) {
     double s[2];
     CK(cudaMemcpyAsync(s, h.norm2.p, sizeof(s), cudaMemcpyDeviceToHost, h.stream));
@@ -1431,7 +1558,7 @@ lbm_status gradient_steady(lbm_handle& h, const double* w, const lbm_adjoint_opt
         CK(cudaEventRecord(e2, h.stream));
         while (st.steps < cap) {
             const int64_t chunk = std::min(check, cap - st.steps);
-            for (int64_t i = 0; i < chunk; ++i) adjoint_step(h, st, h.record.as<float>(), i == chunk - 1);
+            adjoint_run(h, st, h.record.as<float>(), 0, chunk, true, h.t);
             const double nrm = read_norm(h) / st.scale;
             resid = nrm / n0;
             if (resid <= o.tolerance) {
@@ -1538,20 +1665,13 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
         // records of states [s0, e0), then their transposed steps in reverse
         auto reverse_span = [&](int64_t s0, int64_t e0, int64_t seg_start) {
             CK(cudaEventRecord(ef0, h.stream));
-            for (int64_t t = s0; t < e0; ++t) {
-                float* r = rec + (size_t)(t - s0) * rec_stride;
-                if (t + 1 < e0) {
-                    step(h, nullptr, r, stage);
-                    ++recomputed;
-                } else {
-                    inspect(h, nullptr, r, stage);
-                }
-            }
+            run_passes(h, e0 - s0, true, nullptr, rec, (int64_t)rec_stride, stage, nullptr);
+            recomputed += e0 - s0 - 1;
             CK(cudaEventRecord(ef1, h.stream));
             CK(cudaEventRecord(ea0, h.stream));
-            for (int64_t t = e0 - 1; t >= s0; --t)
-                adjoint_step(h, st, rec + (size_t)(t - s0) * rec_stride, t == seg_start, t,
-                             stage && t >= 1 ? &sp : nullptr, rec_planes);
+            // (state 0 is not part of the average)
+            adjoint_run(h, st, rec + (size_t)(e0 - 1 - s0) * rec_stride, (int64_t)rec_stride, e0 - s0, s0 == seg_start,
+                        e0 - 1, stage ? &sp : nullptr, stage ? e0 - std::max<int64_t>(s0, 1) : 0, rec_planes);
             CK(cudaEventRecord(ea1, h.stream));
             CK(cudaEventSynchronize(ea1));
             float a1 = 0, a2 = 0;
@@ -1579,8 +1699,8 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
                 CK(cudaEventCreate(&es1));
                 CK(cudaEventRecord(es0, h.stream));
                 const int64_t last = start + ((end - 1 - start) / KR) * KR;  // the last span's first state
-                for (int64_t t = start; t <= last; ++t) {
-                    if ((t - start) % KR == 0) {
+                for (int64_t t = start; t <= last; t += KR) {
+                    {
                         Checkpoint sc;
                         sc.buf = std::make_unique<DevBuf>();
                         const size_t ab = h.array_bytes(h.storage);
@@ -1591,8 +1711,8 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
                         sub.push_back(std::move(sc));
                     }
                     if (t < last) {
-                        step(h, nullptr, nullptr);
-                        ++recomputed;
+                        run_passes(h, KR, false, nullptr, nullptr, 0, false, nullptr);
+                        recomputed += KR;
                     }
                 }
                 CK(cudaEventRecord(es1, h.stream));
@@ -1703,10 +1823,9 @@ lbm_status gradient_binomial(lbm_handle& h, const double* w, const lbm_adjoint_o
             store(x.b);
         } else if (x.kind == RevolveAction::ADVANCE) {
             need(h.t == x.a);
-            for (int64_t t = x.a; t < x.b; ++t) {
-                prev_pending = h.pending;
-                step(h, d + t, nullptr);
-            }
+            if (x.b - x.a > 1) run_passes(h, x.b - x.a - 1, false, d + x.a, nullptr, 0, false, nullptr);
+            prev_pending = h.pending;
+            step(h, d + x.b - 1, nullptr);
         } else {
             need(false);
         }
@@ -1770,7 +1889,7 @@ lbm_status gradient_binomial(lbm_handle& h, const double* w, const lbm_adjoint_o
                 case RevolveAction::ADVANCE:
                     need(h.t == x.a);
                     mark(0);
-                    for (int64_t t = x.a; t < x.b; ++t) step(h, nullptr, nullptr);
+                    run_passes(h, x.b - x.a, false, nullptr, nullptr, 0, false, nullptr);
                     recomputed += x.b - x.a;
                     break;
                 case RevolveAction::REVERSE: {
