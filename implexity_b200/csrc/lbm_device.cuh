@@ -265,13 +265,15 @@ __device__ __forceinline__ void port_transpose(const PortMap& P, float (&v)[Q]) 
     for (int q = 0; q < Q; ++q) in[q] = v[q];
     const uint32_t um = P.unknown_mask;
 #pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        float acc = (um & (1u << k)) ? 0.f : in[k];
+    for (int k = 0; k < Q; ++k)
+        if (um & (1u << k)) v[k] = 0.f;
+    // row by row: one test per population instead of one per entry
 #pragma unroll
-        for (int r = 0; r < Q; ++r)
-            if (um & (1u << r)) acc = fmaf(P.jac[r][k], in[r], acc);
-        v[k] = acc;
-    }
+    for (int r = 0; r < Q; ++r)
+        if (um & (1u << r)) {
+#pragma unroll
+            for (int k = 0; k < Q; ++k) v[k] = fmaf(P.jac[r][k], in[r], v[k]);
+        }
 }
 
 // ------------------------------------------------------------------ extrapolating ports
@@ -566,13 +568,28 @@ __device__ __forceinline__ double dotc_d(int q, const double (&v)[3]) {
     return s;
 }
 
+// c_q . v summed up from zero (the 16-bit collision's order of operations).
 template <int Q>
-__device__ __forceinline__ float dotc(int q, const float (&v)[3]) {
+__device__ __forceinline__ float dotc0(int q, const float (&v)[3]) {
     using L = Lat<Q>;
     float s = 0.f;
     if (L::cx(q)) s += L::cx(q) * v[0];
     if (L::cy(q)) s += L::cy(q) * v[1];
     if (L::cz(q)) s += L::cz(q) * v[2];
+    return s;
+}
+
+// c_q . v for q >= 1, from the first nonzero component on (a sum that starts
+// at zero costs an addition per direction: 0 + x is not x for x = -0).
+template <int Q>
+__device__ __forceinline__ float dotc(int q, const float (&v)[3]) {
+    using L = Lat<Q>;
+    const int c[3] = {L::cx(q), L::cy(q), L::cz(q)};
+    const int first = c[0] ? 0 : (c[1] ? 1 : 2);
+    float s = c[first] > 0 ? v[first] : -v[first];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        if (d > first && c[d]) s = c[d] > 0 ? s + v[d] : s - v[d];
     return s;
 }
 
@@ -627,9 +644,9 @@ __device__ __forceinline__ Macro collide_fused(float (&v)[Q], float alpha, const
     const float kp = 1.f - 0.5f * om, km = 1.f - 0.5f * omm;
     const float hp = 0.5f * (1.f - om), hm = 0.5f * (1.f - omm);
     const float rho = M.rho;
-    const float usq15 = 1.5f * (M.u[0] * M.u[0] + M.u[1] * M.u[1] + M.u[2] * M.u[2]);
-    const float uf3 = 3.f * (M.u[0] * M.F[0] + M.u[1] * M.F[1] + M.u[2] * M.F[2]);
-    float dproj[MAX_PROJ];
+    [[maybe_unused]] const float usq15 = 1.5f * (M.u[0] * M.u[0] + M.u[1] * M.u[1] + M.u[2] * M.u[2]);
+    [[maybe_unused]] const float uf3 = 3.f * (M.u[0] * M.F[0] + M.u[1] * M.F[1] + M.u[2] * M.F[2]);
+    [[maybe_unused]] float dproj[MAX_PROJ];
     if constexpr (COLL == CK_MRT) {
         // y = f - eq + src/2 of the rest population (g or g/w form)
         const float w0 = SC ? 1.f : L::w(0);
@@ -640,49 +657,98 @@ __device__ __forceinline__ Macro collide_fused(float (&v)[Q], float alpha, const
     }
     float rem = rp;  // mass left for the rest population
     if constexpr (COLL != CK_MRT) {
-        // Pair relaxation with the cell's constants folded:
-        //   P' = hp S + w [E0 + A cu^2 + 9 kp cu cf],  E0 = om (rp - rho 1.5 u^2) - kp 3 u.F,  A = 4.5 om rho
-        //   D' = hm D + w [G cu + 3 km cf],              G = 3 om_odd rho
-        // (the equilibrium and source terms of the MRT branch, regrouped).
-        const float E0 = fmaf(om, fmaf(-rho, usq15, rp), -kp * uf3);
-        const float A = 4.5f * om * rho, G = 3.f * omm * rho;
-        const float K9 = 9.f * kp, K3 = 3.f * km;
-        // MRT_BULK: the bulk moment Eb = sum_i w_i b_i y_i of y = f - eq + src/2,
-        // b_i = |c_i|^2 - 1 (zero on the axis directions); per pair
-        // y_p = S/2 - w [e0 + 4.5 cu (rho cu - cf)], e0 = rp - 1.5 rho u^2 + 1.5 u.F
-        float Eb = 0.f, e0 = 0.f;
-        if constexpr (COLL == CK_MRT_BULK) {
-            const float w0 = SC ? 1.f : L::w(0);
-            const float y0 = v[0] - w0 * (rp - rho * usq15) - 0.5f * w0 * uf3;
-            Eb = -(SC ? L::w(0) : 1.f) * y0;
-            e0 = fmaf(-rho, usq15, rp) + 0.5f * uf3;
-        }
-#pragma unroll
-        for (int k = 0; k < NP; ++k) {
-            const int i = k + 1, o = opp<Q>(i);
-            const float cu = dotc<Q>(i, M.u);
-            const float cf = dotc<Q>(i, M.F);
+        [[maybe_unused]] float Eb = 0.f;  // MRT_BULK: the bulk moment of y = f - eq + src/2
+        if constexpr (SC) {
+            // Pair relaxation in (f - w)/w with the cell's constants folded:
+            //   P' = hp S + E0 + A cu^2 + 9 kp cu cf,  E0 = om (rp - rho 1.5 u^2) - kp 3 u.F,  A = 4.5 om rho
+            //   D' = hm D + G cu + 3 km cf,              G = 3 om_odd rho
+            // (the equilibrium and source terms of the MRT branch, regrouped).  A 16-bit
+            // state rounds every value every step, so another order of these operations
+            // gives another trajectory, off by the storage's noise: the order stays.
+            const float E0 = fmaf(om, fmaf(-rho, usq15, rp), -kp * uf3);
+            const float A = 4.5f * om * rho, G = 3.f * omm * rho;
+            const float K9 = 9.f * kp, K3 = 3.f * km;
+            // MRT_BULK: the bulk moment Eb = sum_i w_i b_i y_i of y = f - eq + src/2,
+            // b_i = |c_i|^2 - 1 (zero on the axis directions); per pair
+            // y_p = S/2 - w [e0 + 4.5 cu (rho cu - cf)], e0 = rp - 1.5 rho u^2 + 1.5 u.F
+            float e0 = 0.f;
             if constexpr (COLL == CK_MRT_BULK) {
-                const int c2 = L::cx(i) * L::cx(i) + L::cy(i) * L::cy(i) + L::cz(i) * L::cz(i);
-                if (c2 != 1) {  // folded after unrolling
-                    const float wy = SC ? 1.f : L::w(i);
-                    const float yp = fmaf(-wy, fmaf(4.5f * cu, fmaf(rho, cu, -cf), e0), 0.5f * S[k]);
-                    Eb = fmaf((SC ? 2.f * L::w(i) : 2.f) * (float)(c2 - 1), yp, Eb);
+                const float y0 = v[0] - 1.f * (rp - rho * usq15) - 0.5f * 1.f * uf3;
+                Eb = -L::w(0) * y0;
+                e0 = fmaf(-rho, usq15, rp) + 0.5f * uf3;
+            }
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                const int i = k + 1, o = opp<Q>(i);
+                const float cu = dotc0<Q>(i, M.u);
+                const float cf = dotc0<Q>(i, M.F);
+                if constexpr (COLL == CK_MRT_BULK) {
+                    const int c2 = L::cx(i) * L::cx(i) + L::cy(i) * L::cy(i) + L::cz(i) * L::cz(i);
+                    if (c2 != 1) {  // folded after unrolling
+                        const float yp = fmaf(-1.f, fmaf(4.5f * cu, fmaf(rho, cu, -cf), e0), 0.5f * S[k]);
+                        Eb = fmaf(2.f * L::w(i) * (float)(c2 - 1), yp, Eb);
+                    }
+                }
+                const float tp = fmaf(cu * cf, K9, fmaf(cu * cu, A, E0));
+                const float tm = fmaf(cu, G, cf * K3);
+                const float Pp = fmaf(hp, S[k], tp), Dm = fmaf(hm, D[k], tm);
+                v[i] = Pp + Dm;
+                v[o] = Pp - Dm;
+                rem = fmaf(-2.f * L::w(i), Pp, rem);
+            }
+        } else {
+            // Pair relaxation (the equilibrium and source terms of the MRT branch,
+            // regrouped): with A = 4.5 om rho, G = 3 om_odd rho and the vectors
+            //   g = A u + 9 kp F,  h = G u + 3 km F
+            //   P' = hp S + w [E0 + (c.u)(c.g)],  E0 = om rp - (u.g) / 3
+            //   D' = hm D + w c.h
+            // The step is bound by instruction issue; taking the products with the
+            // vectors once per cell instead of c.u, c.F and their four products per
+            // pair leaves three to six operations per pair besides its sums.
+            const float A = 4.5f * om * rho, G = 3.f * omm * rho;
+            const float K9 = 9.f * kp, K3 = 3.f * km;
+            float gv[3], hv[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                gv[d] = fmaf(A, M.u[d], K9 * M.F[d]);
+                hv[d] = fmaf(G, M.u[d], K3 * M.F[d]);
+            }
+            const float ug = fmaf(M.u[2], gv[2], fmaf(M.u[1], gv[1], M.u[0] * gv[0]));
+            const float E0 = fmaf(om, rp, -(1.f / 3.f) * ug);
+            // MRT_BULK: the bulk moment Eb = sum_i b_i y_i of y = f - eq + src/2, b_i =
+            // |c_i|^2 - 1; the moments of eq and src are closed forms (sum w b = 0,
+            // sum w b c_a c_b = 2/9 delta_ab): Eb = sum_i b_i g_i - rho u.u + u.F
+            if constexpr (COLL == CK_MRT_BULK) {
+                Eb = -v[0];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) Eb = fmaf(M.u[d], fmaf(-rho, M.u[d], M.F[d]), Eb);
+#pragma unroll
+                for (int k = 0; k < NP; ++k) {
+                    const int i = k + 1;
+                    const int c2 = L::cx(i) * L::cx(i) + L::cy(i) * L::cy(i) + L::cz(i) * L::cz(i);
+                    if (c2 != 1) Eb = fmaf((float)(c2 - 1), S[k], Eb);  // folded after unrolling
                 }
             }
-            const float tp = fmaf(cu * cf, K9, fmaf(cu * cu, A, E0));
-            const float tm = fmaf(cu, G, cf * K3);
-            float Pp, Dm;
-            if constexpr (SC) {
-                Pp = fmaf(hp, S[k], tp);
-                Dm = fmaf(hm, D[k], tm);
-            } else {
-                Pp = fmaf(tp, L::w(i), hp * S[k]);
-                Dm = fmaf(tm, L::w(i), hm * D[k]);
+            // the weight of each class (|c|^2 = 1, 2, 3) enters the vectors
+#pragma unroll
+            for (int cls = 1; cls <= (Q == 19 ? 2 : 3); ++cls) {
+                float wc = 1.f;
+#pragma unroll
+                for (int i = 1; i <= NP; ++i)
+                    if (L::cx(i) * L::cx(i) + L::cy(i) * L::cy(i) + L::cz(i) * L::cz(i) == cls) wc = L::w(i);
+                const float e = wc * E0;
+                const float gc[3] = {wc * gv[0], wc * gv[1], wc * gv[2]}, hc[3] = {wc * hv[0], wc * hv[1], wc * hv[2]};
+#pragma unroll
+                for (int k = 0; k < NP; ++k) {
+                    const int i = k + 1, o = opp<Q>(i);
+                    if (L::cx(i) * L::cx(i) + L::cy(i) * L::cy(i) + L::cz(i) * L::cz(i) != cls) continue;
+                    const float Pp = fmaf(hp, S[k], fmaf(dotc<Q>(i, M.u), dotc<Q>(i, gc), e));
+                    const float Dm = fmaf(hm, D[k], dotc<Q>(i, hc));
+                    v[i] = Pp + Dm;
+                    v[o] = Pp - Dm;
+                    rem = fmaf(-2.f, Pp, rem);
+                }
             }
-            v[i] = Pp + Dm;
-            v[o] = Pp - Dm;
-            rem = fmaf(SC ? -2.f * L::w(i) : -2.f, Pp, rem);
         }
         if constexpr (COLL == CK_MRT_BULK) {
             // rank-one bulk correction: v_i -= (s_bulk - omega) Eb w_i b_i / |b|^2_W,
@@ -878,20 +944,24 @@ __device__ __forceinline__ float collide_vjp(float (&gb)[Q], float rp, const flo
     constexpr int NP = L::NPAIR;
     const float rho = 1.f + rp;
     const float s = 1.f + 0.5f * alpha;
-    float F[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) F[d] = rho * (P.a[d] - alpha * u[d]);
     // weighted moments of gb, pair by pair; the pair sums and differences are
     // kept for the output pass, which applies the TRT part of the transpose
     // (gb - R^T gb per pair: (1 - om)/2 sm +- (1 - omm)/2 df)
-    float M0 = L::w(0) * gb[0];
+    // The cotangents of a cell are nearly one value (a pressure objective's
+    // most of all) and the collision conserves mass, C^T 1 = 1: the transpose
+    // acts on the differences from the rest population's, r + C^T (gb - r).
+    // That takes the cancellations out of the moments: the FP32 bias of a step
+    // in the mass mode falls from 1.9e-8 to under 1e-9 of r, the alpha
+    // cotangent's error by a factor of ten.
+    const float r = gb[0];
+    float M0 = 0.f;
     float M1[3] = {0.f, 0.f, 0.f}, M2[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     float SM[NP], DF[NP];
-    float g0 = (1.f - om) * gb[0];  // the rest population's output, less rho_bar
+    float g0 = 0.f;  // the rest population's output, less rho_bar and r
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
         const int i = k + 1, o = opp<Q>(i);
-        const float sm = gb[i] + gb[o], df = gb[i] - gb[o];
+        const float sm = fmaf(-2.f, r, gb[i] + gb[o]), df = gb[i] - gb[o];
         SM[k] = sm;
         DF[k] = df;
         const float w = L::w(i);
@@ -913,103 +983,115 @@ __device__ __forceinline__ float collide_vjp(float (&gb)[Q], float rp, const flo
         if (c0 && c2) M2[4] = fmaf(w * c0 * c2, sm, M2[4]);
         if (c1 && c2) M2[5] = fmaf(w * c1 * c2, sm, M2[5]);
     }
-    float Z0 = om * M0, H0 = (1.f - 0.5f * om) * M0;
-    float Z1[3], H1[3], Z2[6], H2[6];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        Z1[d] = omm * M1[d];
-        H1[d] = (1.f - 0.5f * omm) * M1[d];
-    }
-#pragma unroll
-    for (int e = 0; e < 6; ++e) {
-        Z2[e] = om * M2[e];
-        H2[e] = (1.f - 0.5f * om) * M2[e];
-    }
-    float bulk_c = 0.f;  // MRT_BULK: the bulk correction's coefficient
-    if constexpr (COLL == CK_MRT_BULK) {
-        // the bulk correction folded: b_i = |c_i|^2 - 1, |b|^2_W = 2/3,
-        // sum_i w_i b_i = 0 and sum_i w_i b_i c_ia c_ib = 2/9 delta_ab on both lattices
-        float e = -L::w(0) * gb[0];
-#pragma unroll
-        for (int k = 0; k < NP; ++k) {
-            const int i = k + 1;
-            const int c2 = L::cx(i) * L::cx(i) + L::cy(i) * L::cy(i) + L::cz(i) * L::cz(i);
-            if (c2 != 1) e = fmaf(L::w(i) * (float)(c2 - 1), SM[k], e);  // folded after unrolling
-        }
-        bulk_c = P.proj_rate[0] * e * 1.5f;
-        const float c = bulk_c;
-        g0 += c;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            Z2[d] = fmaf(c, 2.f / 9.f, Z2[d]);
-            H2[d] = fmaf(-0.5f * c, 2.f / 9.f, H2[d]);
-        }
-    }
-    float cproj[MAX_PROJ];  // MRT: the rank-one corrections' coefficients
-    if constexpr (COLL == CK_MRT) {
-#pragma unroll
-        for (int p = 0; p < MAX_PROJ; ++p) {
-            cproj[p] = 0.f;
-            if (p < P.n_proj) {
-                float e = 0.f;
-#pragma unroll
-                for (int i = 0; i < Q; ++i) e = fmaf(P.proj_left[p][i], gb[i], e);
-                const float c = P.proj_rate[p] * e;
-                cproj[p] = c;
-                g0 = fmaf(-c, P.proj_right[p][0], g0);
-                Z0 = fmaf(c, P.proj_m0[p], Z0);
-                H0 = fmaf(-0.5f * c, P.proj_m0[p], H0);
-#pragma unroll
-                for (int e2 = 0; e2 < 6; ++e2) {
-                    Z2[e2] = fmaf(c, P.proj_m2[p][e2], Z2[e2]);
-                    H2[e2] = fmaf(-0.5f * c, P.proj_m2[p][e2], H2[e2]);
-                }
-            }
-        }
-    }
-    // Z2 u, H2 u, H2 F (symmetric 3x3 stored xx yy zz xy xz yz)
+    // The cotangents of (rho, u, F) and the Brinkman chain, collected.  With
+    //   e  = 9 M2 u - 3 M0 u,  ea = 9 M2 a - 3 M0 a
+    // (the equilibrium's and the source's second-order terms) and hz, ho = 1 -
+    // om/2, 1 - omm/2, the force F = rho (a - alpha u) makes every term a
+    // multiple of M1, e and ea:
+    //   F_bar = 3 ho M1 + hz e
+    //   u_bar = rho [(om - 2 hz alpha) e + 3 (omm - ho alpha) M1 + hz ea]
+    //   rho_bar = om M0 + om/2 u.e + 3 omm u.M1 + F_bar.(a - alpha u) - m_bar.(s u - a/2)
+    //   m_bar = u_bar / (rho s)
+    // An even MRT correction adds its moments D0, D2 to those of the relaxed
+    // part and takes half of them from the source's: with e' = 9 D2 u - 3 D0 u
+    // and ea' likewise, F_bar -= e'/2, u_bar += rho [(1 + alpha) e' - ea'/2],
+    // rho_bar += D0 + u.e'/2.
+    const float hz = 1.f - 0.5f * om, ho = 1.f - 0.5f * omm;
+    const bool forced = P.a[0] != 0.f || P.a[1] != 0.f || P.a[2] != 0.f;  // the same for every cell
+    // symmetric 3x3 stored xx yy zz xy xz yz
     auto mul = [](const float (&S)[6], const float* v, float* out) {
         out[0] = S[0] * v[0] + S[3] * v[1] + S[4] * v[2];
         out[1] = S[3] * v[0] + S[1] * v[1] + S[5] * v[2];
         out[2] = S[4] * v[0] + S[5] * v[1] + S[2] * v[2];
     };
-    float Z2u[3], H2u[3], H2F[3];
-    mul(Z2, u, Z2u);
-    mul(H2, u, H2u);
-    mul(H2, F, H2F);
-    const float usq = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
-    float rho_bar = Z0 * (1.f - 1.5f * usq) + 3.f * (u[0] * Z1[0] + u[1] * Z1[1] + u[2] * Z1[2]) +
-                    4.5f * (u[0] * Z2u[0] + u[1] * Z2u[1] + u[2] * Z2u[2]);
-    float ub[3], Fb[3];
+    float e[3];
+    mul(M2, u, e);
+    const float M03 = 3.f * M0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) e[d] = fmaf(9.f, e[d], -M03 * u[d]);
+    float bulk_c = 0.f;     // MRT_BULK: the bulk correction's coefficient
+    float cproj[MAX_PROJ];  // MRT: the rank-one corrections' coefficients
+    float D0 = 0.f, ep[3] = {0.f, 0.f, 0.f}, eap[3] = {0.f, 0.f, 0.f};
+    if constexpr (COLL == CK_MRT_BULK) {
+        // the bulk correction folded: b_i = |c_i|^2 - 1, |b|^2_W = 2/3,
+        // sum_i w_i b_i = 0 and sum_i w_i b_i c_ia c_ib = 2/9 delta_ab on both lattices
+        float b = 0.f;
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+            const int i = k + 1;
+            const int c2 = L::cx(i) * L::cx(i) + L::cy(i) * L::cy(i) + L::cz(i) * L::cz(i);
+            if (c2 != 1) b = fmaf(L::w(i) * (float)(c2 - 1), SM[k], b);  // folded after unrolling
+        }
+        bulk_c = P.proj_rate[0] * b * 1.5f;
+        g0 += bulk_c;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            ep[d] = 2.f * bulk_c * u[d];
+            eap[d] = 2.f * bulk_c * P.a[d];
+        }
+    }
+    if constexpr (COLL == CK_MRT) {
+        float D2[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int p = 0; p < MAX_PROJ; ++p) {
+            cproj[p] = 0.f;
+            if (p < P.n_proj) {
+                float b = 0.f;
+#pragma unroll
+                for (int i = 1; i < Q; ++i) b = fmaf(P.proj_left[p][i], gb[i] - r, b);
+                const float c = P.proj_rate[p] * b;
+                cproj[p] = c;
+                g0 = fmaf(-c, P.proj_right[p][0], g0);
+                D0 = fmaf(c, P.proj_m0[p], D0);
+#pragma unroll
+                for (int e2 = 0; e2 < 6; ++e2) D2[e2] = fmaf(c, P.proj_m2[p][e2], D2[e2]);
+            }
+        }
+        mul(D2, u, ep);
+        mul(D2, P.a, eap);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            ep[d] = fmaf(9.f, ep[d], -3.f * D0 * u[d]);
+            eap[d] = fmaf(9.f, eap[d], -3.f * D0 * P.a[d]);
+        }
+    }
+    const float ce = fmaf(-2.f * hz, alpha, om), cm1 = 3.f * fmaf(-ho, alpha, omm), ho3 = 3.f * ho;
+    float Fb[3], ur[3];  // F_bar and u_bar / rho
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        ub[d] = rho * (3.f * Z1[d] + 9.f * Z2u[d] - 3.f * u[d] * Z0) + 9.f * H2F[d] - 3.f * F[d] * H0;
-        Fb[d] = 3.f * H1[d] + 9.f * H2u[d] - 3.f * u[d] * H0;
+        Fb[d] = fmaf(hz, e[d], ho3 * M1[d]);
+        ur[d] = fmaf(ce, e[d], cm1 * M1[d]);
+        if constexpr (COLL == CK_MRT_BULK || COLL == CK_MRT) {
+            Fb[d] = fmaf(-0.5f, ep[d], Fb[d]);
+            ur[d] = fmaf(1.f + alpha, ep[d], ur[d]);
+        }
     }
-    float abar = 0.f;
+    if (forced) {
+        float ea[3];
+        mul(M2, P.a, ea);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        rho_bar += Fb[d] * (P.a[d] - alpha * u[d]);
-        abar -= rho * Fb[d] * u[d];
-        ub[d] -= rho * alpha * Fb[d];
+        for (int d = 0; d < 3; ++d) {
+            ur[d] = fmaf(hz, fmaf(9.f, ea[d], -M03 * P.a[d]), ur[d]);
+            if constexpr (COLL == CK_MRT_BULK || COLL == CK_MRT) ur[d] = fmaf(-0.5f, eap[d], ur[d]);
+        }
     }
+    auto dot = [](const float* x, const float* y) { return fmaf(x[2], y[2], fmaf(x[1], y[1], x[0] * y[0])); };
+    const float fu = dot(Fb, u), wu = dot(ur, u);
+    float rho_bar = fmaf(om, fmaf(0.5f, dot(u, e), M0), 3.f * omm * dot(u, M1)) - fmaf(alpha, fu, wu);
+    if constexpr (COLL == CK_MRT_BULK || COLL == CK_MRT) rho_bar += fmaf(0.5f, dot(u, ep), D0);
     const float inv_s = __fdividef(1.f, s);
-    const float inv = __fdividef(inv_s, rho);
     float mb[3];
-    float sbar = 0.f;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        mb[d] = ub[d] * inv;
-        rho_bar -= ub[d] * (s * u[d] - 0.5f * P.a[d]) * inv;
-        sbar -= ub[d] * u[d] * inv_s;
-    }
-    abar += 0.5f * sbar;
+    for (int d = 0; d < 3; ++d) mb[d] = ur[d] * inv_s;
+    if (forced) rho_bar += dot(Fb, P.a) + 0.5f * dot(mb, P.a);
+    // d/d alpha: -rho F_bar.u through F, -u_bar.u / (2 s) through u
+    const float abar = -rho * fmaf(0.5f * inv_s, wu, fu);
     // output, times k: gb - R^T gb + rho_bar + c . mb, pair by pair (with
     // the MRT corrections, which are even: the same for i and opp(i)); the
     // scale k of the stored cotangent enters the few per-cell coefficients
     // instead of every population
     const float hp = 0.5f * (1.f - om) * k, hm = 0.5f * (1.f - omm) * k;
-    const float kr = k * rho_bar, kbulk = k * bulk_c;
+    const float kr = k * (rho_bar + r), kbulk = k * bulk_c;
     float kmb[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) kmb[d] = k * mb[d];
@@ -1547,25 +1629,34 @@ __device__ __forceinline__ constexpr int rund_aligned(int q) {
     return d < 0 ? d + V : d;
 }
 
+// min of three in one instruction (NaN operands are ignored, as by fminf)
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 // Minimum population f = w + g (or w (1 + g/w) in 16-bit storage units) of
 // one cell: the minimum is taken per weight class (|c|^2) first.
 template <int Q, int SC>
 __device__ __forceinline__ float min_population(const float (&v)[Q]) {
     using L = Lat<Q>;
-    float m[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        const int k = (L::cx(q) != 0) + (L::cy(q) != 0) + (L::cz(q) != 0);
-        m[k] = fminf(m[k], v[q]);
-    }
     float mn = INFINITY;
 #pragma unroll
     for (int k = 0; k < (Q == 19 ? 3 : 4); ++k) {
         float w = 0.f;  // the class weight (a compile-time constant after unrolling)
+        float m = INFINITY, kept = 0.f;
+        bool has = false;
 #pragma unroll
-        for (int r = 0; r < Q; ++r)
-            if ((L::cx(r) != 0) + (L::cy(r) != 0) + (L::cz(r) != 0) == k) w = L::w(r);
-        mn = fminf(mn, SC ? w * (1.f + m[k]) : w + m[k]);
+        for (int q = 0; q < Q; ++q) {
+            if ((L::cx(q) != 0) + (L::cy(q) != 0) + (L::cz(q) != 0) != k) continue;
+            w = L::w(q);
+            if (has) m = min3(m, kept, v[q]);
+            else kept = v[q];
+            has = !has;
+        }
+        if (has) m = fminf(m, kept);
+        mn = fminf(mn, SC ? w * (1.f + m) : w + m);
     }
     return mn;
 }
