@@ -23,7 +23,8 @@ MMA_SOURCE = CSRC / "mma_cpu.cpp"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
-SOURCES = ["lbm_forward.cu", "lbm_adjoint.cu", "lbm_march.cu", "lbm_misc.cu", "lbm_noalloc.cu", "lbm_runtime.cpp"]
+SOURCES = ["lbm_forward.cu", "lbm_adjoint.cu", "lbm_march.cu", "lbm_misc.cu", "lbm_io.cu", "lbm_noalloc.cu",
+           "lbm_runtime.cpp"]
 # The stepping kernels' instances compile as one unit per lattice and collision
 # (LBM_PART: 10 * lattice + CollKind), in parallel with the rest.  (nvcc's own
 # --split-compile makes them spill: 0 -> 108 bytes in the FP32 forward step,
@@ -32,6 +33,7 @@ PARTS = {"lbm_forward.cu": [190, 191, 192, 270, 271, 272], "lbm_adjoint.cu": [19
          "lbm_march.cu": [190, 192, 270, 272]}
 UNITS = [(src, part) for part in (191, 271, 190, 270, 192, 272, None) for src in SOURCES
          if part is None or part in PARTS.get(src, ())]
+UNITS.sort(key=lambda u: u[0] != "lbm_misc.cu")  # the longest one first
 
 
 def nvcc() -> str:

@@ -163,6 +163,7 @@ struct DesignArgs {
     float* alpha;
     float* den;
     float* slope;
+    const int* refuse;       // nonzero: the raw design was refused, keep the last map (nullptr: off)
     // sensitivity
     const float* phibar;
     const float* abar;
@@ -223,6 +224,11 @@ cudaError_t launch_seed_lam(int Q, int lstorage, const Geometry& G, void* lam, c
 // (left in the port cells' slots) into the neighbours' slots.
 cudaError_t launch_nee_move(int lstorage, void* lam, int64_t n, int Q, const uint32_t* cells, int64_t count,
                             int64_t nb_off, cudaStream_t s);
+// in (FP64) -> out (FP32); unit: a value outside [0, 1] sets *bad.
+cudaError_t launch_narrow(const double* in, float* out, int64_t n, int unit, int* bad, cudaStream_t s);
+// f[k cells][Q] (FP64) -> g = f - w in planes of stride n; a non-finite value of a solid cell sets the flag.
+cudaError_t launch_cells_to_planes(int Q, const double* f, float* g, int64_t n, int64_t k, const double* w,
+                                   const uint8_t* cls, int* solid_nonfinite, cudaStream_t s);
 cudaError_t launch_design_map(const DesignArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_sens_scale(const DesignArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_filter_transpose(const DesignArgs& a, int grid, cudaStream_t s);

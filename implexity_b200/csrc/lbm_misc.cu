@@ -449,6 +449,7 @@ __device__ __forceinline__ bool shifted(const Geometry& G, int64_t x, int dx, in
 
 // DesignMap::map + resistance (design.rs:199-216, 284-286).
 __global__ void __launch_bounds__(BLOCK) k_design_map(DesignArgs a) {
+    if (a.refuse && *a.refuse) return;
     for (int64_t x = (int64_t)blockIdx.x * BLOCK + threadIdx.x; x < a.G.n; x += (int64_t)gridDim.x * BLOCK) {
         const uint8_t c = a.cls[x];
         float phi, den = 1.f, slope = 0.f;

@@ -6,13 +6,18 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <charconv>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "../../include/lbm_b200.h"
@@ -322,20 +327,74 @@ void reconstruct(const HostLat& L, const PortSpec& p, const double a[3], const d
 }
 
 // ------------------------------------------------------------ device buffers
+// Checkpoints come from one stream-ordered pool per device instead of
+// cudaMalloc / cudaFree on every gradient: on a shared host those took 20 to
+// 100 ms for a horizon gradient's sixteen 320 MB states and varied with the
+// neighbours' load.  Freed states stay in the pool up to POOL_KEEP bytes, for
+// the next gradient of any handle (the frees are ordered on the owner's
+// stream, the driver orders a reuse on another); a failing allocation gives
+// them back first.
+constexpr uint64_t POOL_KEEP = 8ull << 30;
+
+cudaMemPool_t state_pool(int device) {
+    static std::mutex mu;
+    static std::map<int, cudaMemPool_t> pools;
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = pools.find(device);
+    if (it != pools.end()) return it->second;
+    cudaMemPool_t pool = nullptr;
+    int ok = 0;
+    if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, device) == cudaSuccess && ok) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        uint64_t keep = POOL_KEEP;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)
+            pool = nullptr;
+        cudaGetLastError();
+    }
+    return pools[device] = pool;
+}
+
+// Gives the pool's unused memory back to the device.
+void trim_pool() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    if (cudaMemPool_t pool = state_pool(dev)) {
+        cudaDeviceSynchronize();  // pending frees reach the pool
+        cudaMemPoolTrimTo(pool, 0);
+    }
+}
+
+// Bytes the pool holds and nobody uses.
+size_t pool_idle(int device) {
+    uint64_t held = 0, used = 0;
+    cudaMemPool_t pool = state_pool(device);
+    if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+        return 0;
+    return held > used ? (size_t)(held - used) : 0;
+}
+
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
     int64_t* counter = nullptr;
+    cudaStream_t pooled = nullptr;  // the stream that frees a buffer of the pool
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { reset(); }
     void reset() {
         if (p) {
-            cudaFree(p);
+            if (pooled) cudaFreeAsync(p, pooled);
+            else cudaFree(p);
             if (counter) *counter -= (int64_t)bytes;
         }
         p = nullptr;
+        pooled = nullptr;
         bytes = 0;
     }
     // exactly b bytes (releases a larger buffer)
@@ -347,15 +406,135 @@ struct DevBuf {
         if (p && bytes >= b) return;
         reset();
         counter = ctr;
-        CK(cudaMalloc(&p, b));
+        cudaError_t e = cudaMalloc(&p, b);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            trim_pool();
+            e = cudaMalloc(&p, b);
+        }
+        if (e != cudaSuccess) p = nullptr;
+        CK(e);
         bytes = b;
         if (counter) *counter += (int64_t)b;
+    }
+    // b bytes of the device's pool, used and freed in the order of stream s
+    void alloc_pooled(size_t b, int64_t* ctr, int device, cudaStream_t s) {
+        reset();
+        if (cudaMemPool_t pool = state_pool(device)) {
+            if (cudaMallocFromPoolAsync(&p, b, pool, s) == cudaSuccess) {
+                pooled = s;
+                bytes = b;
+                counter = ctr;
+                if (counter) *counter += (int64_t)b;
+                return;
+            }
+            cudaGetLastError();
+            p = nullptr;
+        }
+        alloc(b, ctr);
     }
     template <typename T>
     T* as() const {
         return static_cast<T*>(p);
     }
 };
+
+// Pinned staging memory for what a call takes from and gives to the host,
+// leased for the call from a process-wide list: a new handle's first call does
+// not page-lock memory again (10 to 50 ms for 16 MB on a shared host).  The
+// list keeps at most four buffers (PIN_CAP bytes each at most) while handles
+// exist and is emptied with the last one; a lease belongs to one call, so
+// threads with handles of their own do not meet in a buffer.
+constexpr int64_t PIN_CAP = 32 << 20;
+
+struct PinList {
+    std::mutex mu;
+    std::vector<std::pair<void*, size_t>> idle;
+    int64_t handles = 0;
+};
+PinList& pin_list() {
+    static PinList* list = new PinList;  // not destroyed: handles may outlive static objects
+    return *list;
+}
+void pin_handles(int by) {
+    PinList& L = pin_list();
+    std::lock_guard<std::mutex> lock(L.mu);
+    L.handles += by;
+    if (L.handles > 0) return;
+    for (auto& b : L.idle) cudaFreeHost(b.first);
+    L.idle.clear();
+}
+
+struct PinLease {
+    void* p = nullptr;
+    size_t bytes = 0;
+    explicit PinLease(size_t want) {
+        size_t size = 64 << 10;
+        while (size < want) size *= 2;
+        PinList& L = pin_list();
+        {
+            std::lock_guard<std::mutex> lock(L.mu);
+            for (size_t i = 0; i < L.idle.size(); ++i)
+                if (L.idle[i].second >= size) {
+                    p = L.idle[i].first;
+                    bytes = L.idle[i].second;
+                    L.idle.erase(L.idle.begin() + (std::ptrdiff_t)i);
+                    return;
+                }
+        }
+        CK(cudaMallocHost(&p, size));
+        bytes = size;
+    }
+    PinLease(const PinLease&) = delete;
+    PinLease& operator=(const PinLease&) = delete;
+    // (a lease ends after its call's last synchronisation: no copy is in flight)
+    ~PinLease() {
+        PinList& L = pin_list();
+        std::lock_guard<std::mutex> lock(L.mu);
+        L.idle.emplace_back(p, bytes);
+        if (L.idle.size() > 4) {  // the smallest goes
+            size_t at = 0;
+            for (size_t i = 1; i < L.idle.size(); ++i)
+                if (L.idle[i].second < L.idle[at].second) at = i;
+            cudaFreeHost(L.idle[at].first);
+            L.idle.erase(L.idle.begin() + (std::ptrdiff_t)at);
+        }
+    }
+    float* floats() const { return static_cast<float*>(p); }
+};
+size_t pin_bytes(int64_t values) { return (size_t)std::min<int64_t>(values * 4, PIN_CAP); }
+
+// fn(begin, end) over [0, n), in chunks that helper threads share with the
+// calling one where the work is worth it.  The caller takes chunks itself and
+// waits only for chunks in progress: a helper that is not scheduled in time
+// (the caller's own thread pool may still spin on every core) finds nothing
+// left and leaves without touching fn.
+template <typename F>
+void parallel_range(int64_t n, F&& fn) {
+    constexpr int64_t CHUNK = 1 << 16;
+    struct Job {
+        std::atomic<int64_t> next{0}, done{0};
+    };
+    const int64_t chunks = (n + CHUNK - 1) / CHUNK;
+    const auto take = [n, chunks](Job& job, F& f) {
+        for (int64_t c; (c = job.next.fetch_add(1)) < chunks; job.done.fetch_add(1)) f(c * CHUNK, std::min(n, (c + 1) * CHUNK));
+    };
+    if (chunks < 4) {
+        if (n > 0) fn((int64_t)0, n);
+        return;
+    }
+    const auto job = std::make_shared<Job>();
+    const int64_t helpers = std::min<int64_t>({7, (int64_t)std::thread::hardware_concurrency() - 1, chunks / 2 - 1});
+    for (int64_t k = 0; k < helpers; ++k) {
+        try {
+            std::thread([job, take, &fn] { take(*job, fn); }).detach();
+        } catch (const std::system_error&) {  // no more threads
+            break;
+        }
+    }
+    take(*job, fn);
+    while (job->done.load() < chunks) std::this_thread::yield();
+}
 
 size_t storage_bytes(int s) { return s == LBM_STORE_F32 ? 4 : 2; }
 
@@ -372,6 +551,8 @@ struct AdjState;
 }  // namespace
 
 struct lbm_handle {
+    lbm_handle() { pin_handles(1); }
+    ~lbm_handle() { pin_handles(-1); }
     // --- normalised problem
     int Q = 19, coll = LBM_BGK, storage = LBM_STORE_F32;
     bool collision_fp64 = false;  // FP64 collision arithmetic on FP32 storage
@@ -398,7 +579,6 @@ struct lbm_handle {
     DevBuf pop, mask, alpha, phi, raw, den, slope, cls_d, fixed_d, offsets_d, ports_d, partial, counter, diag;
     DevBuf lam, record, abar, abar_final, phibar, scale, grad, norm2, sums, scratch, errflag;
     DevBuf omega_cell, tau_state, tau_bar;
-    DevBuf march;  // partial records of the passes of one launch, and its barrier counter
     AdjState* slab_adj = nullptr;  // x-slab steady adjoint in progress (lbm_slab_adjoint_begin)
     int lam_storage = LBM_STORE_F32;
     // --- ports: normalised specs with their signals; pulsatile ports keep one
@@ -441,6 +621,10 @@ struct lbm_handle {
     int64_t global_fluid = -1, global_inlet = -1, global_outlet = -1;
     int64_t t = 0;
     std::string err;
+
+    // device words: the bounded waits' error flag, the flag set by the checks of
+    // a call's values, the barrier counter of a run of passes (a line each)
+    int* word(int k) const { return errflag.as<int>() + 64 * k; }
 
     int64_t n() const { return G.n; }
     // One array (Q planes plus front and back padding) of the given storage,
@@ -915,7 +1099,7 @@ void validate_and_build(lbm_handle& h, const lbm_problem_t& p) {
     h.pop.alloc(2 * h.array_bytes(h.storage), ctr);
     h.mask.alloc((size_t)(n + CELL_PAD) * 4, ctr);
     h.alpha.alloc((size_t)(n + CELL_PAD) * 4, ctr);
-    h.errflag.alloc(sizeof(int), ctr);
+    h.errflag.alloc(3 * 64 * sizeof(int), ctr);
     h.phi.alloc((size_t)n * 4, ctr);
     h.raw.alloc((size_t)n * 4, ctr);
     h.den.alloc((size_t)n * 4, ctr);
@@ -944,7 +1128,7 @@ void validate_and_build(lbm_handle& h, const lbm_problem_t& p) {
         CK(cudaMemcpyAsync(h.ports_d.p, maps.data(), maps.size() * sizeof(PortMap), cudaMemcpyHostToDevice,
                            h.stream));
     CK(cudaMemsetAsync(h.counter.p, 0, 2 * sizeof(unsigned), h.stream));
-    CK(cudaMemsetAsync(h.errflag.p, 0, sizeof(int), h.stream));
+    CK(cudaMemsetAsync(h.errflag.p, 0, h.errflag.bytes, h.stream));
     CK(cudaMemsetAsync(h.pop.p, 0, h.pop.bytes, h.stream));
     CK(cudaStreamSynchronize(h.stream));
     h.time_average = p.time_average != 0;
@@ -1047,7 +1231,6 @@ int64_t march_chunk(lbm_handle& h, bool stage) {
     const int64_t per = march_scratch(h.n(), h.sms, stage);
     return std::max<int64_t>(8, std::min<int64_t>(128, (8 << 20) / per));
 }
-constexpr size_t MARCH_HEAD = 256;  // the barrier counter, ahead of the partial records
 
 // `passes` forward passes from the current state; with inspect_last the last
 // one is load-only (inspect), else every pass steps.  diag / record / stage
@@ -1067,7 +1250,8 @@ void run_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* diag
     ensure_port_maps(h, h.t + passes);
     const int64_t chunk = march_chunk(h, stage != nullptr);
     const int64_t scratch = chunk * march_scratch(h.n(), h.sms, stage != nullptr);
-    h.march.alloc(MARCH_HEAD + (size_t)scratch, &h.device_bytes);
+    DevBuf partial;  // the passes' partial records
+    if (diag || stage) partial.alloc_pooled((size_t)scratch, &h.device_bytes, h.device, h.stream);
     for (int64_t i = 0; i < passes;) {
         const int64_t k = std::min(chunk, passes - i);
         const bool inspects = inspect_last && i + k == passes;
@@ -1085,8 +1269,8 @@ void run_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* diag
         g.port_stride = h.pulsatile ? h.n_ports : 0;
         g.record_stride = record_stride;
         g.diag = diag ? diag + i : nullptr;
-        g.bar = h.march.as<unsigned>();
-        g.scratch = h.march.as<char>() + MARCH_HEAD;
+        g.bar = reinterpret_cast<unsigned*>(h.word(2));
+        g.scratch = partial.p;
         g.scratch_bytes = scratch;
         CK(launch_march_forward(h.Q, coll_kernel(h), h.storage, g, h.stream));
         const int64_t steps = k - (inspects ? 1 : 0);
@@ -1207,7 +1391,7 @@ lbm_status run_admitted(lbm_handle& h, int64_t steps, lbm_diag_t* out, int64_t K
             Checkpoint c;
             c.buf = std::make_unique<DevBuf>();
             const size_t ab = h.array_bytes(h.storage);
-            c.buf->alloc(ab, ctr);
+            c.buf->alloc_pooled(ab, ctr, h.device, h.stream);
             CK(cudaMemcpyAsync(c.buf->p, h.pop_array(h.cur), ab, cudaMemcpyDeviceToDevice, h.stream));
             c.t = h.t;
             c.pending = h.pending;
@@ -1223,10 +1407,9 @@ lbm_status run_admitted(lbm_handle& h, int64_t steps, lbm_diag_t* out, int64_t K
     std::vector<StepDiag>& hd = h.last_trajectory;
     hd.resize((size_t)steps + 1);
     CK(cudaMemcpyAsync(hd.data(), d, hd.size() * sizeof(StepDiag), cudaMemcpyDeviceToHost, h.stream));
-    CK(cudaStreamSynchronize(h.stream));
+    check_errflag(h);
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, h.ev0, h.ev1));
-    check_errflag(h);
     if (averages) finish_time_average(h, steps);
     return admit(h, hd, out, ms);
 }
@@ -1316,6 +1499,65 @@ DesignArgs design_args(lbm_handle& h) {
     return a;
 }
 
+// ------------------------------------------------------------ host arrays
+// A call's FP64 results pass through pinned FP32 staging in pieces of at most
+// PIN_CAP bytes: the copy runs at the link's rate and the conversion, which
+// first touches the pages of the caller's new array, on several threads (one
+// thread took 5 ms for 4.2M cells; an FP64 copy into untouched pages 7.6 ms).
+// in (host FP64) -> dev (FP32), narrowed on the device in pieces of at most
+// IO_CAP bytes; with `unit` a value outside [0, 1] sets flags[0].
+constexpr int64_t IO_CAP = 64 << 20;
+
+// (from the pool: a new handle's first call allocates nothing)
+void io_buffer(lbm_handle& h, DevBuf& io, int64_t values) {
+    io.alloc_pooled((size_t)std::min<int64_t>(values * 8, IO_CAP), &h.device_bytes, h.device, h.stream);
+}
+
+void upload(lbm_handle& h, const double* in, float* dev, int64_t n, bool unit) {
+    DevBuf buf;
+    io_buffer(h, buf, n);
+    double* io = buf.as<double>();
+    const int64_t piece = IO_CAP / 8;
+    for (int64_t x = 0; x < n; x += piece) {
+        const int64_t k = std::min(piece, n - x);
+        CK(cudaMemcpyAsync(io, in + x, (size_t)k * 8, cudaMemcpyHostToDevice, h.stream));
+        CK(launch_narrow(io, dev + x, k, unit ? 1 : 0, h.word(1), h.stream));
+    }
+}
+
+// Reads the flag that the checks of a call set, and clears it.
+bool take_flag(lbm_handle& h) {
+    int bad = 0;
+    CK(cudaMemcpyAsync(&bad, h.word(1), sizeof(int), cudaMemcpyDeviceToHost, h.stream));
+    CK(cudaStreamSynchronize(h.stream));
+    if (bad) CK(cudaMemsetAsync(h.word(1), 0, sizeof(int), h.stream));
+    return bad != 0;
+}
+
+// dev (FP32) -> out (host FP64); returns whether every value is finite.
+bool download(lbm_handle& h, const PinLease& pin, const float* dev, double* out, int64_t n) {
+    float* st = pin.floats();
+    const int64_t piece = PIN_CAP / 4;
+    std::atomic<bool> finite{true};
+    for (int64_t x = 0; x < n; x += piece) {
+        const int64_t k = std::min(piece, n - x);
+        CK(cudaMemcpyAsync(st, dev + x, (size_t)k * 4, cudaMemcpyDeviceToHost, h.stream));
+        CK(cudaStreamSynchronize(h.stream));
+        parallel_range(k, [&](int64_t b, int64_t e) {
+            bool good = true;
+            for (int64_t i = b; i < e; ++i) {
+                good = good && std::isfinite(st[i]);
+                out[x + i] = st[i];
+            }
+            if (!good) finite = false;
+        });
+    }
+    return finite;
+}
+
+// Cells per piece of an array of `planes` FP32 planes of n cells.
+int64_t plane_piece(int64_t n, int planes) { return std::min(n, PIN_CAP / (4 * planes)); }
+
 // phi_bar -> raw gradient on the device (grad buffer), scaled abar optional.
 void design_transpose(lbm_handle& h, const float* phibar, const float* abar, float abar_scale,
                       const float* abar_final) {
@@ -1404,7 +1646,6 @@ void adjoint_run(lbm_handle& h, AdjState& st, const float* rec, int64_t stride, 
                          i < stage_steps ? stage : nullptr, rec_planes);
         return;
     }
-    h.march.alloc(MARCH_HEAD, &h.device_bytes);
     for (int64_t i = 0; i < count;) {
         const int64_t k = std::min<int64_t>(128, count - i);
         MarchAdjArgs g{};
@@ -1424,7 +1665,7 @@ void adjoint_run(lbm_handle& h, AdjState& st, const float* rec, int64_t stride, 
         g.n_ports = h.n_ports;
         g.port_stride = h.pulsatile && stride ? h.n_ports : 0;
         g.record_stride = stride;
-        g.bar = h.march.as<unsigned>();
+        g.bar = reinterpret_cast<unsigned*>(h.word(2));
         CK(launch_march_adjoint(h.Q, coll_kernel(h), h.lam_storage, g, h.stream));
         h.lcur ^= (int)(k & 1);
         st.scale = st.target;
@@ -1534,14 +1775,8 @@ float next_scale(const lbm_handle& h, double true_norm, float cur) {
 void finish_gradient(lbm_handle& h, const AdjState& st, bool any_adjoint, double* grad) {
     design_transpose(h, h.phibar.as<float>(), any_adjoint ? h.abar.as<float>() : nullptr, 1.f / st.s0,
                      h.abar_final.as<float>());
-    std::vector<float> g((size_t)h.n());
-    CK(cudaMemcpyAsync(g.data(), h.grad.p, g.size() * 4, cudaMemcpyDeviceToHost, h.stream));
-    CK(cudaStreamSynchronize(h.stream));
-    bool finite = true;
-    for (int64_t x = 0; x < h.n(); ++x) {
-        grad[x] = g[x];
-        finite = finite && std::isfinite(g[x]);
-    }
+    const PinLease pin(pin_bytes(h.n()));
+    const bool finite = download(h, pin, h.grad.as<float>(), grad, h.n());
     if (!finite) throw ContractError("Nonfinite LBM sensitivity");
 }
 
@@ -1633,10 +1868,11 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
     // KR steps, then each span once more with its records (scan.rs Every(K)
     // nested in itself; one more recomputed forward).
     int64_t KR = K;
-    h.record.reset();  // sized below from the memory left
     {
         size_t free_b = 0, total_b = 0;
         CK(cudaMemGetInfo(&free_b, &total_b));
+        // the memory left, with what the pool keeps and the record of the last call
+        free_b += pool_idle(h.device) + h.record.bytes;
         const size_t ab = h.array_bytes(h.storage);
         const double ckpt_bytes = (double)((T + K - 1) / K + 2) * (double)ab;
         double budget = 0.8 * ((double)free_b - ckpt_bytes) - (double)(1ull << 30);
@@ -1712,7 +1948,7 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
                         Checkpoint sc;
                         sc.buf = std::make_unique<DevBuf>();
                         const size_t ab = h.array_bytes(h.storage);
-                        sc.buf->alloc(ab, ctr);
+                        sc.buf->alloc_pooled(ab, ctr, h.device, h.stream);
                         CK(cudaMemcpyAsync(sc.buf->p, h.pop_array(h.cur), ab, cudaMemcpyDeviceToDevice, h.stream));
                         sc.t = h.t;
                         sc.pending = h.pending;
@@ -1807,7 +2043,7 @@ lbm_status gradient_binomial(lbm_handle& h, const double* w, const lbm_adjoint_o
         Checkpoint& c = slots[(size_t)slot];
         if (!c.buf) {
             c.buf = std::make_unique<DevBuf>();
-            c.buf->alloc(ab, ctr);
+            c.buf->alloc_pooled(ab, ctr, h.device, h.stream);
         }
         const char* cur = h.restored ? h.restored : h.pop_array(h.cur);
         CK(cudaMemcpyAsync(c.buf->p, cur, ab, cudaMemcpyDeviceToDevice, h.stream));
@@ -2053,18 +2289,12 @@ lbm_status lbm_info(const lbm_handle* h, lbm_info_t* out) {
 lbm_status lbm_set_design(lbm_handle* h, const double* raw, size_t n) {
     return guarded(h, [&]() {
         check_n(*h, n, (size_t)h->n(), "model:control");
-        std::vector<float> r(n);
-        for (size_t x = 0; x < n; ++x) {
-            double v = raw[x];
-            if (!std::isfinite(v) || v < 0.0 || v > 1.0)
-                throw ContractError("model:control must be a finite shape-matched array in [0,1]");
-            r[x] = (float)v;
-        }
-        CK(cudaMemcpyAsync(h->raw.p, r.data(), n * 4, cudaMemcpyHostToDevice, h->stream));
+        upload(*h, raw, h->raw.as<float>(), (int64_t)n, true);
         DesignArgs a = design_args(*h);
         const int grid = (int)std::min<int64_t>((h->n() + 255) / 256, (int64_t)h->sms * 8);
+        a.refuse = h->word(1);  // a refused design leaves the last one's map in place
         CK(launch_design_map(a, grid, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        if (take_flag(*h)) throw ContractError("model:control must be a finite shape-matched array in [0,1]");
         h->design_set = true;
         h->forward_done = false;
         return LBM_OK;
@@ -2100,15 +2330,9 @@ lbm_status lbm_set_tau(lbm_handle* h, const double* tau, size_t n) {
 lbm_status lbm_get_design(lbm_handle* h, double* phi, double* alpha) {
     return guarded(h, [&]() {
         require_design(*h);
-        std::vector<float> b((size_t)h->n());
-        if (phi) {
-            CK(cudaMemcpy(b.data(), h->phi.p, b.size() * 4, cudaMemcpyDeviceToHost));
-            for (size_t x = 0; x < b.size(); ++x) phi[x] = b[x];
-        }
-        if (alpha) {
-            CK(cudaMemcpy(b.data(), h->alpha.p, b.size() * 4, cudaMemcpyDeviceToHost));
-            for (size_t x = 0; x < b.size(); ++x) alpha[x] = b[x];
-        }
+        const PinLease pin(pin_bytes(h->n()));
+        if (phi) download(*h, pin, h->phi.as<float>(), phi, h->n());
+        if (alpha) download(*h, pin, h->alpha.as<float>(), alpha, h->n());
         return LBM_OK;
     });
 }
@@ -2141,27 +2365,23 @@ lbm_status lbm_set_populations(lbm_handle* h, const double* f, size_t n) {
         const int64_t N = h->n();
         const int Q = h->Q;
         check_n(*h, n, (size_t)(N * Q), "populations");
-        std::vector<float> g((size_t)N * Q);
-        bool solid_nonfinite = false;
-    // x-slab of a larger problem (lbm_create_slab): the owned planes are
-    // [slab_hl, slab_hl + slab_own) of the local grid, the others ghost planes;
-    // responses, seeds and port pressure weights use the whole problem's counts
-    bool slab = false;
-    int32_t slab_hl = 0, slab_hr = 0, slab_own = 0;
-    int64_t global_fluid = -1, global_inlet = -1, global_outlet = -1;
-        for (int64_t x = 0; x < N; ++x) {
-            for (int q = 0; q < Q; ++q) g[(size_t)q * N + x] = (float)(f[x * Q + q] - h->L.w[q]);
-            if (h->cls[x] == 0)  // solid
-                for (int q = 0; q < Q; ++q) solid_nonfinite = solid_nonfinite || !std::isfinite(f[x * Q + q]);
-        }
         ensure_scratch(*h);
-        CK(cudaMemcpyAsync(h->scratch.p, g.data(), g.size() * 4, cudaMemcpyHostToDevice, h->stream));
+        const int64_t piece = std::min<int64_t>(N, IO_CAP / (8 * Q));
+        DevBuf buf;
+        io_buffer(*h, buf, piece * Q);
+        double* io = buf.as<double>();
+        for (int64_t x0 = 0; x0 < N; x0 += piece) {
+            const int64_t k = std::min(piece, N - x0);
+            CK(cudaMemcpyAsync(io, f + x0 * Q, (size_t)(k * Q) * 8, cudaMemcpyHostToDevice, h->stream));
+            CK(launch_cells_to_planes(Q, io, h->scratch.as<float>() + x0, N, k, h->L.w, h->cls_d.as<uint8_t>() + x0,
+                                      h->word(1), h->stream));
+        }
         const int grid = grid_for(*h);
         // both arrays: solid cells keep their populations in either
         for (int k = 0; k < 2; ++k)
             CK(launch_upload_pop(Q, h->storage, h->G, k ? h->popB() : h->popA(), h->mask.as<uint32_t>(),
                                  h->scratch.as<float>(), grid, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        const bool solid_nonfinite = take_flag(*h);
         h->pending = false;
         h->t = 0;
         h->state_valid = true;
@@ -2180,11 +2400,19 @@ lbm_status lbm_get_populations(lbm_handle* h, double* f, size_t n) {
         ensure_scratch(*h);
         CK(launch_canon_pop(Q, h->storage, h->G, h->popA(), h->mask.as<uint32_t>(), ports_at(*h, h->t),
                             h->pending ? 1 : 0, h->scratch.as<float>(), grid_for(*h), h->stream));
-        std::vector<float> g((size_t)N * Q);
-        CK(cudaMemcpyAsync(g.data(), h->scratch.p, g.size() * 4, cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-        for (int64_t x = 0; x < N; ++x)
-            for (int q = 0; q < Q; ++q) f[x * Q + q] = h->L.w[q] + (double)g[(size_t)q * N + x];
+        const int64_t piece = plane_piece(N, Q);
+        const PinLease pin(pin_bytes(piece * Q));
+        float* g = pin.floats();
+        for (int64_t x0 = 0; x0 < N; x0 += piece) {
+            const int64_t k = std::min(piece, N - x0);
+            CK(cudaMemcpy2DAsync(g, (size_t)k * 4, h->scratch.as<float>() + x0, (size_t)N * 4, (size_t)k * 4, (size_t)Q,
+                                 cudaMemcpyDeviceToHost, h->stream));
+            CK(cudaStreamSynchronize(h->stream));
+            parallel_range(k * Q, [&](int64_t b, int64_t e) {
+                for (int64_t x = (b + Q - 1) / Q; x < (e + Q - 1) / Q; ++x)
+                    for (int q = 0; q < Q; ++q) f[(x0 + x) * Q + q] = h->L.w[q] + (double)g[q * k + x];
+            });
+        }
         return LBM_OK;
     });
 }
@@ -2324,20 +2552,30 @@ lbm_status lbm_fields(lbm_handle* h, double* density, double* velocity, double* 
         ensure_scratch(*h);
         double r8[8];
         responses(*h, r8, h->scratch.as<float>());
-        std::vector<float> fl((size_t)N * 4);
-        CK(cudaMemcpyAsync(fl.data(), h->scratch.p, fl.size() * 4, cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
         const double vel = h->dx / h->dt;
         const double unit = vel * vel / 3.0;
-        for (int64_t x = 0; x < N; ++x) {
-            const bool solid = h->cls[x] == 0;
-            // solid cells keep their equilibrium populations: rho = 1, u = 0
-            const double rp = solid ? 0.0 : (double)fl[x];
-            const double rho = (1.0 + rp) * h->density;
-            if (density) density[x] = rho;
-            if (pressure) pressure[x] = (rho - h->density) * unit;
-            if (velocity)
-                for (int d = 0; d < 3; ++d) velocity[3 * x + d] = solid ? 0.0 : (double)fl[(size_t)(d + 1) * N + x] * vel;
+        const int64_t piece = plane_piece(N, 4);
+        const PinLease pin(pin_bytes(piece * 4));
+        float* fl = pin.floats();
+        for (int64_t x0 = 0; x0 < N; x0 += piece) {
+            const int64_t k = std::min(piece, N - x0);
+            CK(cudaMemcpy2DAsync(fl, (size_t)k * 4, h->scratch.as<float>() + x0, (size_t)N * 4, (size_t)k * 4, 4,
+                                 cudaMemcpyDeviceToHost, h->stream));
+            CK(cudaStreamSynchronize(h->stream));
+            parallel_range(k * 4, [&](int64_t b, int64_t e) {
+                for (int64_t i = (b + 3) / 4; i < (e + 3) / 4; ++i) {
+                    const int64_t x = x0 + i;
+                    const bool solid = h->cls[x] == 0;
+                    // solid cells keep their equilibrium populations: rho = 1, u = 0
+                    const double rp = solid ? 0.0 : (double)fl[i];
+                    const double rho = (1.0 + rp) * h->density;
+                    if (density) density[x] = rho;
+                    if (pressure) pressure[x] = (rho - h->density) * unit;
+                    if (velocity)
+                        for (int d = 0; d < 3; ++d)
+                            velocity[3 * x + d] = solid ? 0.0 : (double)fl[(d + 1) * k + i] * vel;
+                }
+            });
         }
         return LBM_OK;
     });
@@ -2754,13 +2992,10 @@ lbm_status lbm_design_vjp(lbm_handle* h, const double* phi_bar, double* out, siz
         check_n(*h, n, (size_t)h->n(), "phi_bar");
         int64_t* ctr = &h->device_bytes;
         h->phibar.alloc(n * 4, ctr);
-        std::vector<float> v(n);
-        for (size_t x = 0; x < n; ++x) v[x] = (float)phi_bar[x];
-        CK(cudaMemcpyAsync(h->phibar.p, v.data(), n * 4, cudaMemcpyHostToDevice, h->stream));
+        const PinLease pin(pin_bytes((int64_t)n));
+        upload(*h, phi_bar, h->phibar.as<float>(), (int64_t)n, false);
         design_transpose(*h, h->phibar.as<float>(), nullptr, 1.f, nullptr);
-        CK(cudaMemcpyAsync(v.data(), h->grad.p, n * 4, cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-        for (size_t x = 0; x < n; ++x) out[x] = v[x];
+        download(*h, pin, h->grad.as<float>(), out, (int64_t)n);
         return LBM_OK;
     });
 }
