@@ -334,7 +334,7 @@ void reconstruct(const HostLat& L, const PortSpec& p, const double a[3], const d
 // the next gradient of any handle (the frees are ordered on the owner's
 // stream, the driver orders a reuse on another); a failing allocation gives
 // them back first.
-constexpr uint64_t POOL_KEEP = 8ull << 30;
+constexpr uint64_t POOL_KEEP = 16ull << 30;
 
 cudaMemPool_t state_pool(int device) {
     static std::mutex mu;
@@ -1376,7 +1376,9 @@ void finish_time_average(lbm_handle& h, int64_t steps);
 // device as well (the stage objective's value, lbm_time_average): the step
 // that reads state t sums its responses into slot t, the final inspection
 // those of the last state.
-lbm_status run_admitted(lbm_handle& h, int64_t steps, lbm_diag_t* out, int64_t K, bool averages = false) {
+// With `record`, the records of every state, record_stride floats apart.
+lbm_status run_admitted(lbm_handle& h, int64_t steps, lbm_diag_t* out, int64_t K, bool averages = false,
+                        float* record = nullptr, int64_t record_stride = 0, bool record_s = false) {
     require_design(h);
     int64_t* ctr = &h.device_bytes;
     h.diag.alloc((size_t)(steps + 1) * sizeof(StepDiag), ctr);
@@ -1399,8 +1401,8 @@ lbm_status run_admitted(lbm_handle& h, int64_t steps, lbm_diag_t* out, int64_t K
         }
         // up to the next checkpoint; the last run ends with the final inspection
         const int64_t e = K > 0 && s / K * K + K < steps ? s / K * K + K : steps + 1;
-        run_passes(h, e - s, e == steps + 1, d + s, nullptr, 0, false,
-                   averages ? h.tsums.as<double>() + (size_t)s * 16 : nullptr);
+        run_passes(h, e - s, e == steps + 1, d + s, record ? record + (size_t)s * record_stride : nullptr,
+                   record_stride, record_s, averages ? h.tsums.as<double>() + (size_t)s * 16 : nullptr);
         s = e;
     }
     CK(cudaEventRecord(h.ev1, h.stream));
@@ -1505,7 +1507,7 @@ DesignArgs design_args(lbm_handle& h) {
 // first touches the pages of the caller's new array, on several threads (one
 // thread took 5 ms for 4.2M cells; an FP64 copy into untouched pages 7.6 ms).
 // in (host FP64) -> dev (FP32), narrowed on the device in pieces of at most
-// IO_CAP bytes; with `unit` a value outside [0, 1] sets flags[0].
+// IO_CAP bytes; with `unit` a value outside [0, 1] sets the handle's flag.
 constexpr int64_t IO_CAP = 64 << 20;
 
 // (from the pool: a new handle's first call allocates nothing)
@@ -1860,7 +1862,16 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
     const int rec_planes = stage ? 10 : 4;
     alloc_adjoint(h, o.lambda_storage);
     int64_t* ctr = &h.device_bytes;
-    const size_t rec_bytes = (size_t)h.n() * rec_planes * sizeof(float);
+    // every record 16-byte aligned (the staged kernels copy its planes in bulk)
+    const size_t rec_stride = ((size_t)h.n() * rec_planes + 3) / 4 * 4;
+    const size_t rec_bytes = rec_stride * sizeof(float);
+    // With the checkpoint interval left to the library, the records of the
+    // whole trajectory are kept where the pool can keep them too (and half of
+    // what is free): the forward sweep writes them as it goes and
+    // nothing is recomputed, which is a quarter to a third of the gradient
+    // (256x128x128 MRT, 200 steps: 90.5 -> 64 ms; 48x24x24, 800 steps: 10.7 -> 7
+    // ms).  The segments stay, as the points where the cotangent is rescaled.
+    DevBuf whole;
     // Records for KR steps.  When a segment's K records do not fit (the
     // caller's record budget, or ~80% of the device memory left after the
     // T/K checkpoints), a second checkpoint level splits each segment into
@@ -1874,17 +1885,26 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
         // the memory left, with what the pool keeps and the record of the last call
         free_b += pool_idle(h.device) + h.record.bytes;
         const size_t ab = h.array_bytes(h.storage);
+        const size_t all = (size_t)(T + 1) * rec_bytes + CELL_PAD * sizeof(float);
+        if (o.checkpoint_every <= 0 && o.record_budget_bytes <= 0 && all <= std::min<size_t>(POOL_KEEP, free_b / 2)) {
+            try {
+                whole.alloc_pooled(all, ctr, h.device, h.stream);
+            } catch (const CudaError&) {  // taken by someone else meanwhile: checkpoints instead
+                cudaGetLastError();
+                whole.reset();
+            }
+        }
         const double ckpt_bytes = (double)((T + K - 1) / K + 2) * (double)ab;
         double budget = 0.8 * ((double)free_b - ckpt_bytes) - (double)(1ull << 30);
         if (o.record_budget_bytes > 0) budget = std::min(budget, (double)o.record_budget_bytes);
-        const int64_t fit = budget > 0 ? (int64_t)(budget / (double)rec_bytes) : 0;
+        const int64_t fit = whole.p ? K : budget > 0 ? (int64_t)(budget / (double)rec_bytes) : 0;
         if (fit < 1) throw ContractError("checkpoint interval needs more record memory than record_budget_bytes");
         // the fewest spans, of equal length: the same recomputation as the
         // longest spans that fit, with less record memory
         const int64_t spans = (K + fit - 1) / fit;
         KR = (K + spans - 1) / spans;
     }
-    h.record.fit(rec_bytes * (size_t)KR + CELL_PAD * sizeof(float), ctr);
+    if (!whole.p) h.record.fit(rec_bytes * (size_t)KR + CELL_PAD * sizeof(float), ctr);
     h.ckpts.clear();
     // forward with checkpoints, then admission (the reference re-runs parts())
     init_state(h);
@@ -1892,13 +1912,13 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
     CK(cudaEventCreate(&ef0));
     CK(cudaEventCreate(&ef1));
     lbm_diag_t dg{};
-    run_admitted(h, T, &dg, K);
+    float* const rec = whole.p ? whole.as<float>() : h.record.as<float>();
+    if (whole.p) run_admitted(h, T, &dg, 0, false, rec, (int64_t)rec_stride, stage);
+    else run_admitted(h, T, &dg, K);
     h.forward_done = true;
     AdjState st;
     const double n0 = seed(h, w, st, nullptr, stage ? 1.0 / (double)T : 1.0);
     const SeedParams sp = stage_seed(h, w, 1.0 / (double)T);
-    float* rec = h.record.as<float>();
-    const size_t rec_stride = (size_t)h.n() * rec_planes;
     int64_t recomputed = 0;
     float ms_fwd = 0, ms_adj = 0;
     if (n0 > 0 || stage) {
@@ -1906,29 +1926,41 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
         CK(cudaEventCreate(&ea0));
         CK(cudaEventCreate(&ea1));
         int64_t peak_sub = 0;
+        // the transposed steps of states [s0, e0) in reverse; their records
+        // follow each other from first_rec on
+        auto transposed_span = [&](const float* first_rec, int64_t s0, int64_t e0, int64_t seg_start) {
+            CK(cudaEventRecord(ea0, h.stream));
+            // (state 0 is not part of the average)
+            adjoint_run(h, st, first_rec + (size_t)(e0 - 1 - s0) * rec_stride, (int64_t)rec_stride, e0 - s0,
+                        s0 == seg_start, e0 - 1, stage ? &sp : nullptr, stage ? e0 - std::max<int64_t>(s0, 1) : 0,
+                        rec_planes);
+            CK(cudaEventRecord(ea1, h.stream));
+            CK(cudaEventSynchronize(ea1));
+            float a2 = 0;
+            CK(cudaEventElapsedTime(&a2, ea0, ea1));
+            ms_adj += a2;
+        };
         // records of states [s0, e0), then their transposed steps in reverse
         auto reverse_span = [&](int64_t s0, int64_t e0, int64_t seg_start) {
             CK(cudaEventRecord(ef0, h.stream));
             run_passes(h, e0 - s0, true, nullptr, rec, (int64_t)rec_stride, stage, nullptr);
             recomputed += e0 - s0 - 1;
             CK(cudaEventRecord(ef1, h.stream));
-            CK(cudaEventRecord(ea0, h.stream));
-            // (state 0 is not part of the average)
-            adjoint_run(h, st, rec + (size_t)(e0 - 1 - s0) * rec_stride, (int64_t)rec_stride, e0 - s0, s0 == seg_start,
-                        e0 - 1, stage ? &sp : nullptr, stage ? e0 - std::max<int64_t>(s0, 1) : 0, rec_planes);
-            CK(cudaEventRecord(ea1, h.stream));
-            CK(cudaEventSynchronize(ea1));
-            float a1 = 0, a2 = 0;
+            transposed_span(rec, s0, e0, seg_start);
+            float a1 = 0;
             CK(cudaEventElapsedTime(&a1, ef0, ef1));
-            CK(cudaEventElapsedTime(&a2, ea0, ea1));
             ms_fwd += a1;
-            ms_adj += a2;
         };
         auto restore = [&](const Checkpoint& c) {
             CK(cudaMemcpyAsync(h.pop_array(h.cur), c.buf->p, c.buf->bytes, cudaMemcpyDeviceToDevice, h.stream));
             h.pending = c.pending;
             h.t = c.t;
         };
+        for (int64_t s0 = whole.p ? (T - 1) / K * K : -1; s0 >= 0; s0 -= K) {
+            transposed_span(rec + (size_t)s0 * rec_stride, s0, std::min(s0 + K, T), s0);
+            // rescale the stored adjoint at segment boundaries
+            st.target = next_scale(h, read_norm(h) / st.scale, st.scale);
+        }
         for (int64_t ci = (int64_t)h.ckpts.size() - 1; ci >= 0; --ci) {
             Checkpoint& c = h.ckpts[ci];
             const int64_t start = c.t, end = std::min(start + K, T);
@@ -1983,7 +2015,7 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
     }
     cudaEventDestroy(ef0);
     cudaEventDestroy(ef1);
-    int64_t peak = (int64_t)h.record.bytes + h.peak_extra;
+    int64_t peak = (int64_t)(whole.p ? whole.bytes : h.record.bytes) + h.peak_extra;
     for (auto& c : h.ckpts) peak += (int64_t)c.buf->bytes;
     h.peak_extra = 0;
     h.ckpts.clear();

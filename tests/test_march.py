@@ -129,3 +129,21 @@ def test_pulsatile_run_matches_single_steps(gpu_lib):
     assert rel_l2(g_bin, g_one) <= 2e-5
     # per-state sums in FP32 per cell against FP64 per cell
     assert np.allclose(mean[[0, 3, 4, 5, 6, 7]], acc[[0, 3, 4, 5, 6, 7]], rtol=1e-5)
+
+
+@pytest.mark.parametrize("objective", ["final", "time_average"])
+def test_kept_records_match_recomputed_ones(gpu_lib, objective):
+    """checkpoint_every=0 keeps every state's record where they fit; a record
+    budget makes it checkpoint.  The same records either way, on a grid whose
+    odd cell count leaves a record's end unaligned."""
+    prob = workloads.pulsatile_problem(shape=(9, 7, 5), steps=T, lattice="D3Q19", period_steps=9)
+    w = np.array([0.3, 0.0, 0.0, 1e3, 1e3, 0.0, 1.0, 1e6])
+    with LbmSolver(prob) as s:
+        s.set_design(workloads.uniform_design((9, 7, 5), 3))
+        g, kept = s.gradient(w, mode="horizon", objective=objective)
+        g_ck, ck = s.gradient(w, mode="horizon", objective=objective, record_budget_bytes=1 << 30)
+        g_one, _ = s.gradient(w, mode="horizon", objective=objective, checkpoint_every=1)
+    assert kept.forward_recomputed == 0 and ck.forward_recomputed > 0
+    assert kept.iterations == ck.iterations == T
+    assert rel_l2(g, g_ck) <= 1e-6
+    assert rel_l2(g, g_one) <= 2e-5
