@@ -234,8 +234,7 @@ cudaError_t LBM_PART_NAME(adjoint)(int storage, const AdjArgs& a, cudaStream_t s
     return cudaErrorInvalidValue;
 }
 #else
-cudaError_t launch_adjoint(int Q, int coll, int lstorage, const AdjArgs& a0, int grid, cudaStream_t s) {
-    (void)grid;
+cudaError_t launch_adjoint(int Q, int coll, int lstorage, const AdjArgs& a0, cudaStream_t s) {
     AdjArgs a = a0;
     run_table(Q, a.G, +1, lstorage == ST_F32 ? 4 : 8, a.run0, a.rund);
     if (a.rec_planes != 4 && a.rec_planes != 10) return cudaErrorInvalidValue;

@@ -1357,60 +1357,44 @@ __device__ DiagAcc block_reduce(DiagAcc v) {
     return v;
 }
 
-// Writes one block's partial, and lets the last block to finish combine all
-// partials in a fixed order (deterministic) into *out.  No block waits.
-__device__ void finish_diag(const DiagLocal& loc, StepDiag* out, const Reduce& red) {
-    __shared__ bool last;
-    DiagAcc v;
-    v.mh = loc.mass;
-    v.ml = 0.0;
-    v.eh = loc.exch;
-    v.el = 0.0;
-    v.minf = loc.minf;
-    v.maxu2 = loc.maxu2;
-    v.nf = loc.nf;
-    v = block_reduce(v);
-    if (threadIdx.x == 0) {
-        double* p = red.partial + (size_t)blockIdx.x * 8;
-        p[0] = v.mh;
-        p[1] = v.ml;
-        p[2] = v.eh;
-        p[3] = v.el;
-        p[4] = v.minf;
-        p[5] = v.maxu2;
-        p[6] = v.nf;
-        __threadfence();
-        unsigned t = atomicAdd(red.counter, 1u);
-        last = (t == gridDim.x - 1);
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+// FP64 sum of per-thread FP32 partial sums.
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(FULL, v, off);
+    return v;
+}
+
+// A warp's share of a pass's admission record; k_reduce_partials combines the
+// warps' of many passes at once.  (The last block of a step used to combine
+// the blocks' partials: two FP64 block reductions and a fence, 3 to 4 us in
+// the tail of every step.)
+__device__ __forceinline__ void store_partial(const DiagLocal& acc, StepPartial* out) {
+    const double mass = warp_sum((double)acc.mass), exch = warp_sum((double)acc.exch);
+    const float mn = warp_min(acc.minf), mx = warp_max(acc.maxu2);
+    const bool nf = __any_sync(FULL, acc.nf);
+    if ((threadIdx.x & 31) == 0) {
+        out->mass = mass;
+        out->exch = exch;
+        out->min_f = mn;
+        out->max_u2 = mx;
+        out->nonfinite = nf;
     }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    DiagAcc acc;
-    acc.init();
-    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-        const double* p = red.partial + (size_t)b * 8;
-        DiagAcc o;
-        o.mh = __ldcg(p + 0);
-        o.ml = __ldcg(p + 1);
-        o.eh = __ldcg(p + 2);
-        o.el = __ldcg(p + 3);
-        o.minf = (float)__ldcg(p + 4);
-        o.maxu2 = (float)__ldcg(p + 5);
-        o.nf = (int)__ldcg(p + 6);
-        acc.merge(o);
-    }
-    acc = block_reduce(acc);
-    if (threadIdx.x == 0) {
-        out->mass_hi = acc.mh;
-        out->mass_lo = acc.ml;
-        out->exch_hi = acc.eh;
-        out->exch_lo = acc.el;
-        out->min_f = acc.minf;
-        out->max_u2 = acc.maxu2;
-        out->nonfinite = acc.nf;
-        *red.counter = 0;
-        __threadfence();
+}
+__device__ __forceinline__ void store_response_partial(const double (&r)[8], double* out) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const double s = warp_sum(r[k]);
+        if ((threadIdx.x & 31) == 0) out[k] = s;
     }
 }
 

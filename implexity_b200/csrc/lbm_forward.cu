@@ -16,12 +16,12 @@
 // Compiled once per lattice and collision (LBM_PART) for the kernels, and once
 // without it for the entry point.
 namespace lbm {
-cudaError_t forward_190(int storage, const FwdArgs& a, cudaStream_t s);
-cudaError_t forward_191(int storage, const FwdArgs& a, cudaStream_t s);
-cudaError_t forward_192(int storage, const FwdArgs& a, cudaStream_t s);
-cudaError_t forward_270(int storage, const FwdArgs& a, cudaStream_t s);
-cudaError_t forward_271(int storage, const FwdArgs& a, cudaStream_t s);
-cudaError_t forward_272(int storage, const FwdArgs& a, cudaStream_t s);
+cudaError_t forward_190(int storage, const FwdArgs& a, cudaStream_t s, uint32_t* warps);
+cudaError_t forward_191(int storage, const FwdArgs& a, cudaStream_t s, uint32_t* warps);
+cudaError_t forward_192(int storage, const FwdArgs& a, cudaStream_t s, uint32_t* warps);
+cudaError_t forward_270(int storage, const FwdArgs& a, cudaStream_t s, uint32_t* warps);
+cudaError_t forward_271(int storage, const FwdArgs& a, cudaStream_t s, uint32_t* warps);
+cudaError_t forward_272(int storage, const FwdArgs& a, cudaStream_t s, uint32_t* warps);
 
 #ifdef LBM_PART
 namespace {
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(TPB, (Q == 19 ? 3 : 2)) k_forward(FwdArgs a) {
                         for (int q = 0; q < Q; ++q) v[q] *= (float)(1.0 / L::wd(q));
                     }
                 }
-                const float mn = a.diag ? min_population<Q, SC>(v) : 0.f;
+                const float mn = a.partial ? min_population<Q, SC>(v) : 0.f;
                 float S[6];
                 if (RSP || (a.record && a.record_s)) {
                     // second moments of g: the stage seeds of the adjoint, the dissipation
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(TPB, (Q == 19 ? 3 : 2)) k_forward(FwdArgs a) {
                     }
                     rsum[7] += (double)r6[5];
                 }
-                if (a.diag) {
+                if (a.partial) {
                     acc.mass += M.rp;
                     acc.exch += exch;
                     acc.minf = fminf(acc.minf, mn);
@@ -225,20 +225,15 @@ __global__ void __launch_bounds__(TPB, (Q == 19 ? 3 : 2)) k_forward(FwdArgs a) {
             }
         }
     }
-    if (a.diag) finish_diag(acc, a.diag, a.red);
-    if constexpr (RSP) {
-        Sums<8> t;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            t.h[k] = rsum[k];
-            t.l[k] = 0.0;
-        }
-        finish_sums<8>(t, a.stage, a.red2);
+    if (warp > 0) {
+        const uint32_t w = blockIdx.x * CONSUMER_WARPS + (uint32_t)(warp - 1);
+        if (a.partial) store_partial(acc, a.partial + w);
+        if constexpr (RSP) store_response_partial(rsum, a.rpartial + (size_t)w * 8);
     }
 }
 
 template <int Q, int COLL, typename T, int AL, int RSP, int DP>
-cudaError_t run_forward_rs(const FwdArgs& a, cudaStream_t s) {
+cudaError_t run_forward_rs(const FwdArgs& a, cudaStream_t s, uint32_t* warps) {
     constexpr size_t smem = pipe_bytes<FwdStage<Q, T>, ring_depth<FwdStage<Q, T>, T>()>();
     static bool attr = false;
     if (!attr) {
@@ -247,20 +242,21 @@ cudaError_t run_forward_rs(const FwdArgs& a, cudaStream_t s) {
         attr = true;
     }
     const int grid = persistent_grid((const void*)k_forward<Q, COLL, T, AL, RSP, DP>, a.G.n, smem, TPB, TILE);
+    if (warps) *warps = (uint32_t)grid * CONSUMER_WARPS;
     k_forward<Q, COLL, T, AL, RSP, DP><<<grid, TPB, smem, s>>>(a);
     return cudaGetLastError();
 }
 
 template <int Q, int COLL, typename T, int AL>
-cudaError_t run_forward_al(const FwdArgs& a, cudaStream_t s) {
+cudaError_t run_forward_al(const FwdArgs& a, cudaStream_t s, uint32_t* warps) {
     if (a.dp_collision) {
         // FP64 collision arithmetic exists for FP32 storage only
         if constexpr (std::is_same<T, float>::value)
-            return a.stage ? run_forward_rs<Q, COLL, T, AL, 1, 1>(a, s) : run_forward_rs<Q, COLL, T, AL, 0, 1>(a, s);
+            return a.rpartial ? run_forward_rs<Q, COLL, T, AL, 1, 1>(a, s, warps) : run_forward_rs<Q, COLL, T, AL, 0, 1>(a, s, warps);
         else
             return cudaErrorInvalidValue;
     }
-    return a.stage ? run_forward_rs<Q, COLL, T, AL, 1, 0>(a, s) : run_forward_rs<Q, COLL, T, AL, 0, 0>(a, s);
+    return a.rpartial ? run_forward_rs<Q, COLL, T, AL, 1, 0>(a, s, warps) : run_forward_rs<Q, COLL, T, AL, 0, 0>(a, s, warps);
 }
 
 // The run offsets are compile-time constants when every run table entry
@@ -275,14 +271,14 @@ bool table_is_aligned(const int32_t* rund) {
 }
 
 template <int Q, int COLL, typename T>
-cudaError_t run_forward(const FwdArgs& a, cudaStream_t s) {
-    return table_is_aligned<Q, T, -1>(a.rund) ? run_forward_al<Q, COLL, T, 1>(a, s) : run_forward_al<Q, COLL, T, 0>(a, s);
+cudaError_t run_forward(const FwdArgs& a, cudaStream_t s, uint32_t* warps) {
+    return table_is_aligned<Q, T, -1>(a.rund) ? run_forward_al<Q, COLL, T, 1>(a, s, warps) : run_forward_al<Q, COLL, T, 0>(a, s, warps);
 }
 
 }  // namespace
 
-cudaError_t LBM_PART_NAME(forward)(int storage, const FwdArgs& a, cudaStream_t s) {
-    LBM_STORAGE_DISPATCH(storage, T, return run_forward<LBM_PART / 10, LBM_PART % 10, T>(a, s))
+cudaError_t LBM_PART_NAME(forward)(int storage, const FwdArgs& a, cudaStream_t s, uint32_t* warps) {
+    LBM_STORAGE_DISPATCH(storage, T, return run_forward<LBM_PART / 10, LBM_PART % 10, T>(a, s, warps))
     return cudaErrorInvalidValue;
 }
 #else
@@ -307,8 +303,7 @@ void run_table(int Q, const Geometry& G, int dir, int vec, int64_t* run0, int32_
     }
 }
 
-cudaError_t launch_forward(int Q, int coll, int storage, const FwdArgs& a0, int grid, cudaStream_t s) {
-    (void)grid;
+cudaError_t launch_forward(int Q, int coll, int storage, const FwdArgs& a0, cudaStream_t s, uint32_t* warps) {
     FwdArgs a = a0;
     run_table(Q, a.G, -1, storage == ST_F32 ? 4 : 8, a.run0, a.rund);
     // every bulk copy needs 16-byte aligned addresses: refuse to launch otherwise
@@ -317,8 +312,8 @@ cudaError_t launch_forward(int Q, int coll, int storage, const FwdArgs& a0, int 
         !staged_aligned(a.alpha, nullptr, 0, 4) || (a.bulk_store && !staged_aligned(a.dst, nullptr, 0, es)))
         return cudaErrorMisalignedAddress;
     if (Q == 19)
-        return coll == CK_MRT ? forward_191(storage, a, s) : coll == CK_MRT_BULK ? forward_192(storage, a, s) : forward_190(storage, a, s);
-    return coll == CK_MRT ? forward_271(storage, a, s) : coll == CK_MRT_BULK ? forward_272(storage, a, s) : forward_270(storage, a, s);
+        return coll == CK_MRT ? forward_191(storage, a, s, warps) : coll == CK_MRT_BULK ? forward_192(storage, a, s, warps) : forward_190(storage, a, s, warps);
+    return coll == CK_MRT ? forward_271(storage, a, s, warps) : coll == CK_MRT_BULK ? forward_272(storage, a, s, warps) : forward_270(storage, a, s, warps);
 }
 #endif
 

@@ -22,6 +22,13 @@ enum StoreKind { ST_F32 = 0, ST_F16 = 1, ST_BF16 = 2 };
 // the bulk moment of the Gram-Schmidt basis (b = |c|^2 - 1), folded at compile time
 enum CollKind { CK_PAIRS = 0, CK_MRT = 1, CK_MRT_BULK = 2 };
 
+// One warp's share of a pass's admission record.
+struct StepPartial {
+    double mass, exch;
+    float min_f, max_u2;
+    int32_t nonfinite, pad;
+};
+
 struct FwdArgs {
     Geometry G;
     Physics P;
@@ -31,18 +38,15 @@ struct FwdArgs {
     const float* alpha;
     const PortMap* ports;
     int32_t apply_ports;     // the stored state still needs the port reconstruction
-    StepDiag* diag;          // per-state admission output (nullptr: off)
-    Reduce red;
+    StepPartial* partial;    // the pass's admission record, one partial per warp (nullptr: off)
     float* record;           // (rho-1, ux, uy, uz) planes (nullptr: off)
     int32_t record_s;        // also record the six second moments of g (planes 4..9)
     int32_t collide;         // 0: only load/diag/record (no collision, no store)
     int32_t bulk_store;      // full tiles leave through bulk stores (planes 16-byte aligned)
     uint32_t step;           // absolute step index (seeds the stochastic rounding)
     int* err;                // set when a bounded wait gave up
-    // response sums of the state the step reads (16 doubles: 8 compensated
-    // sums; nullptr: off), with their own reduction scratch
-    double* stage;
-    Reduce red2;
+    // response sums of the state the step reads, 8 per warp (nullptr: off)
+    double* rpartial;
     const float* phi;        // design density (response 5)
     SeedParams sp;           // unit conversions of the responses (w unused)
     // staged pull runs: element offset of each direction's 16-byte aligned
@@ -82,17 +86,10 @@ struct AdjArgs {
     const float* omega_cell; // per-cell relaxation rate 1/tau (BGK; nullptr: the uniform rate of P)
 };
 
-// One warp's share of a pass's admission record (k_march_forward).
-struct StepPartial {
-    double mass, exch;
-    float min_f, max_u2;
-    int32_t nonfinite, pad;
-};
-
 // A run of forward passes in one cooperative launch (lbm_march.cu): pass 0
 // reads a.src, the passes write a.dst and dst1 in turn.  a.record, diag and
-// a.stage (the response sums of every pass) point at the first pass's slot;
-// a.apply_ports holds for pass 0, the later ones apply every port.
+// stage (the response sums of every pass) point at the first pass's slot;
+// a.partial and a.rpartial are set by the launcher; a.apply_ports holds for pass 0, the later ones apply every port.
 struct MarchFwdArgs {
     FwdArgs a;
     void* dst1;
@@ -102,10 +99,9 @@ struct MarchFwdArgs {
     int32_t port_stride;    // maps from one pass to the next (0: the same)
     int64_t record_stride;  // floats from one pass's record to the next
     StepDiag* diag;         // one per pass (nullptr: off)
-    void* scratch;          // march_scratch() bytes per pass when diag or a.stage is set
+    double* stage;          // 16 doubles per pass: 8 compensated sums (nullptr: off)
+    void* scratch;          // march_scratch() bytes per pass when diag or stage is set
     int64_t scratch_bytes;
-    StepPartial* partial;   // set by the launcher
-    double* rpartial;
     unsigned* bar;          // barrier counter
 };
 
@@ -186,8 +182,15 @@ void set_thread_error(const char* msg);
 
 cudaError_t launch_init(int Q, int storage, const Geometry& G, const Physics& P, void* pop, const uint32_t* mask,
                         int64_t c_begin, int64_t c_end, cudaStream_t s);  // cells [c_begin, c_end)
-cudaError_t launch_forward(int Q, int coll, int storage, const FwdArgs& a, int grid, cudaStream_t s);
-cudaError_t launch_adjoint(int Q, int coll, int lstorage, const AdjArgs& a, int grid, cudaStream_t s);
+// *warps: the partials the step writes (a.partial, a.rpartial).
+cudaError_t launch_forward(int Q, int coll, int storage, const FwdArgs& a, cudaStream_t s, uint32_t* warps = nullptr);
+// Combines the warps' partials of `passes` passes (stride apart), in a fixed
+// order, into diag[pass] and stage[16 * pass] (either may be nullptr).
+cudaError_t launch_reduce_partials(const StepPartial* part, const double* rpart, uint32_t warps, uint32_t stride,
+                                   int passes, StepDiag* diag, double* stage, cudaStream_t s);
+cudaError_t launch_adjoint(int Q, int coll, int lstorage, const AdjArgs& a, cudaStream_t s);
+// Bytes of partials one pass of a grid of n cells needs at most, and warps.
+int64_t pass_warps(int64_t n, int sms);
 // Bytes of MarchFwdArgs::scratch one pass of a grid of n cells needs.
 int64_t march_scratch(int64_t n, int sms, bool stage);
 cudaError_t launch_march_forward(int Q, int coll, int storage, const MarchFwdArgs& g, cudaStream_t s);

@@ -105,23 +105,6 @@ __device__ __forceinline__ bool grid_wait(const unsigned* bar, unsigned target, 
     }
 }
 
-__device__ __forceinline__ float warp_min(float v) {
-    float r;
-    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
-}
-__device__ __forceinline__ float warp_max(float v) {
-    float r;
-    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
-}
-// FP64 sum of per-thread FP32 partial sums.
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(FULL, v, off);
-    return v;
-}
-
 __device__ __forceinline__ void copy_ports(PortMap* to, const PortMap* from, int n) {
     const float* s = reinterpret_cast<const float*>(from);
     float* d = reinterpret_cast<float*>(to);
@@ -141,7 +124,6 @@ __global__ void __launch_bounds__(MT, (Q == 19 && !DP && !RSP ? 3 : 2)) k_march_
     const uint32_t stride = gridDim.x * blockDim.x, x0 = blockIdx.x * blockDim.x + threadIdx.x;
     const bool single = n <= stride;  // one cell per thread: its mask and alpha stay in registers
     const uint32_t warps = stride >> 5, warp = x0 >> 5;
-    const int lane = threadIdx.x & 31;
     copy_ports(ports, a.ports, g.n_ports);
     __syncthreads();
     uint32_t m = 0;
@@ -195,7 +177,7 @@ __global__ void __launch_bounds__(MT, (Q == 19 && !DP && !RSP ? 3 : 2)) k_march_
                     for (int q = 0; q < Q; ++q) v[q] *= (float)(1.0 / L::wd(q));
                 }
             }
-            const float mn = g.partial ? min_population<Q, SC>(v) : 0.f;
+            const float mn = a.partial ? min_population<Q, SC>(v) : 0.f;
             float S[6];
             if (RSP || (record && a.record_s)) {
                 float gg[Q];
@@ -225,7 +207,7 @@ __global__ void __launch_bounds__(MT, (Q == 19 && !DP && !RSP ? 3 : 2)) k_march_
                 }
                 rsum[7] += (double)r6[5];
             }
-            if (g.partial) {
+            if (a.partial) {
                 acc.mass += M.rp;
                 acc.exch += exch;
                 acc.minf = fminf(acc.minf, mn);
@@ -246,78 +228,13 @@ __global__ void __launch_bounds__(MT, (Q == 19 && !DP && !RSP ? 3 : 2)) k_march_
             if (g.port_stride) copy_ports(ports, a.ports + (size_t)(pass + 1) * g.port_stride, g.n_ports);
         }
         // the pass's record, while the barrier fills
-        if (g.partial) {
-            const double mass = warp_sum((double)acc.mass), exch = warp_sum((double)acc.exch);
-            const float mn = warp_min(acc.minf), mx = warp_max(acc.maxu2);
-            const bool nf = __any_sync(FULL, acc.nf);
-            if (lane == 0) {
-                StepPartial& p = g.partial[(size_t)pass * warps + warp];
-                p.mass = mass;
-                p.exch = exch;
-                p.min_f = mn;
-                p.max_u2 = mx;
-                p.nonfinite = nf;
-            }
-        }
-        if constexpr (RSP) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const double s = warp_sum(rsum[k]);
-                if (lane == 0) g.rpartial[((size_t)pass * warps + warp) * 8 + k] = s;
-            }
-        }
+        if (a.partial) store_partial(acc, a.partial + (size_t)pass * warps + warp);
+        if constexpr (RSP) store_response_partial(rsum, a.rpartial + ((size_t)pass * warps + warp) * 8);
         if (more) {
             if (threadIdx.x == 0) go = grid_wait(g.bar, (unsigned)(pass + 1) * gridDim.x, a.err);
             __syncthreads();
             if (!go) return;
         }
-    }
-}
-
-// One block per pass: the warps' partials combined in a fixed order.
-__global__ void __launch_bounds__(256) k_march_reduce(const StepPartial* part, const double* rpart, uint32_t warps,
-                                                      StepDiag* out, double* stage) {
-    const size_t pass = blockIdx.x;
-    if (out) {
-        DiagAcc acc;
-        acc.init();
-        for (uint32_t i = threadIdx.x; i < warps; i += blockDim.x) {
-            const StepPartial& p = part[pass * warps + i];
-            DiagAcc o;
-            o.mh = p.mass;
-            o.ml = 0.0;
-            o.eh = p.exch;
-            o.el = 0.0;
-            o.minf = p.min_f;
-            o.maxu2 = p.max_u2;
-            o.nf = p.nonfinite;
-            acc.merge(o);
-        }
-        acc = block_reduce(acc);
-        if (threadIdx.x == 0) {
-            StepDiag& d = out[pass];
-            d.mass_hi = acc.mh;
-            d.mass_lo = acc.ml;
-            d.exch_hi = acc.eh;
-            d.exch_lo = acc.el;
-            d.min_f = acc.minf;
-            d.max_u2 = acc.maxu2;
-            d.nonfinite = acc.nf;
-        }
-    }
-    if (stage) {
-        Sums<8> s;
-        s.init();
-        for (uint32_t i = threadIdx.x; i < warps; i += blockDim.x)
-#pragma unroll
-            for (int k = 0; k < 8; ++k) s.add(k, rpart[(pass * warps + i) * 8 + k]);
-        s = block_reduce_sums<8>(s);
-        if (threadIdx.x == 0)
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                stage[pass * 16 + 2 * k] = s.h[k];
-                stage[pass * 16 + 2 * k + 1] = s.l[k];
-            }
     }
 }
 
@@ -451,25 +368,24 @@ cudaError_t run_march(MarchFwdArgs& g, cudaStream_t s) {
     const uint32_t warps = (uint32_t)(sh.grid * sh.threads / 32);
     const int64_t per_pass = (int64_t)warps * ((g.diag ? sizeof(StepPartial) : 0) + (RSP ? 64 : 0));
     if (per_pass * g.n_pass > g.scratch_bytes) return cudaErrorInvalidValue;
-    g.partial = g.diag ? static_cast<StepPartial*>(g.scratch) : nullptr;
-    g.rpartial = RSP ? reinterpret_cast<double*>(static_cast<char*>(g.scratch) +
-                                                 (g.diag ? (size_t)g.n_pass * warps * sizeof(StepPartial) : 0))
-                     : nullptr;
-    cudaError_t e = launch_cooperative(kernel, sh, g, s);
+    g.a.partial = g.diag ? static_cast<StepPartial*>(g.scratch) : nullptr;
+    g.a.rpartial = RSP ? reinterpret_cast<double*>(static_cast<char*>(g.scratch) +
+                                                   (g.diag ? (size_t)g.n_pass * warps * sizeof(StepPartial) : 0))
+                       : nullptr;
+    const cudaError_t e = launch_cooperative(kernel, sh, g, s);
     if (e != cudaSuccess || !per_pass) return e;
-    k_march_reduce<<<g.n_pass, 256, 0, s>>>(g.partial, g.rpartial, warps, g.diag, RSP ? g.a.stage : nullptr);
-    return cudaGetLastError();
+    return launch_reduce_partials(g.a.partial, g.a.rpartial, warps, warps, g.n_pass, g.diag, g.stage, s);
 }
 
 template <int Q, int COLL, typename T>
 cudaError_t run_march_forward(MarchFwdArgs& g, cudaStream_t s) {
     if (g.a.dp_collision) {
         if constexpr (std::is_same<T, float>::value)
-            return g.a.stage ? run_march<Q, COLL, T, 1, 1>(g, s) : run_march<Q, COLL, T, 0, 1>(g, s);
+            return g.stage ? run_march<Q, COLL, T, 1, 1>(g, s) : run_march<Q, COLL, T, 0, 1>(g, s);
         else
             return cudaErrorInvalidValue;
     }
-    return g.a.stage ? run_march<Q, COLL, T, 1, 0>(g, s) : run_march<Q, COLL, T, 0, 0>(g, s);
+    return g.stage ? run_march<Q, COLL, T, 1, 0>(g, s) : run_march<Q, COLL, T, 0, 0>(g, s);
 }
 
 template <int Q, int COLL, typename T>
@@ -493,10 +409,68 @@ cudaError_t LBM_PART_NAME(march_adjoint)(int storage, MarchAdjArgs& g, cudaStrea
     return cudaErrorInvalidValue;
 }
 #else
+namespace {
+// One block per pass: the warps' partials combined in a fixed order.
+__global__ void __launch_bounds__(256) k_reduce_partials(const StepPartial* part, const double* rpart,
+                                                         uint32_t warps, uint32_t stride, StepDiag* out, double* stage) {
+    const size_t pass = blockIdx.x;
+    if (out) {
+        DiagAcc acc;
+        acc.init();
+        for (uint32_t i = threadIdx.x; i < warps; i += blockDim.x) {
+            const StepPartial& p = part[pass * stride + i];
+            DiagAcc o;
+            o.mh = p.mass;
+            o.ml = 0.0;
+            o.eh = p.exch;
+            o.el = 0.0;
+            o.minf = p.min_f;
+            o.maxu2 = p.max_u2;
+            o.nf = p.nonfinite;
+            acc.merge(o);
+        }
+        acc = block_reduce(acc);
+        if (threadIdx.x == 0) {
+            StepDiag& d = out[pass];
+            d.mass_hi = acc.mh;
+            d.mass_lo = acc.ml;
+            d.exch_hi = acc.eh;
+            d.exch_lo = acc.el;
+            d.min_f = acc.minf;
+            d.max_u2 = acc.maxu2;
+            d.nonfinite = acc.nf;
+        }
+    }
+    if (stage) {
+        Sums<8> s;
+        s.init();
+        for (uint32_t i = threadIdx.x; i < warps; i += blockDim.x)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s.add(k, rpart[(pass * stride + i) * 8 + k]);
+        s = block_reduce_sums<8>(s);
+        if (threadIdx.x == 0)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                stage[pass * 16 + 2 * k] = s.h[k];
+                stage[pass * 16 + 2 * k + 1] = s.l[k];
+            }
+    }
+}
+
+}  // namespace
+
+int64_t pass_warps(int64_t n, int sms) {
+    // eight (consumer) warps per 256 cells, at most 8 blocks per SM
+    return std::min<int64_t>((n + 255) / 256 * 8, (int64_t)sms * 64);
+}
 int64_t march_scratch(int64_t n, int sms, bool stage) {
-    // at most 8 blocks of 256 threads per SM, and a tiny grid's blocks of 128
-    const int64_t warps = std::min<int64_t>((n + 255) / 256 * 8, (int64_t)sms * 64);
-    return warps * (int64_t)(sizeof(StepPartial) + (stage ? 64 : 0));
+    return pass_warps(n, sms) * (int64_t)(sizeof(StepPartial) + (stage ? 64 : 0));
+}
+
+cudaError_t launch_reduce_partials(const StepPartial* part, const double* rpart, uint32_t warps, uint32_t stride,
+                                   int passes, StepDiag* diag, double* stage, cudaStream_t s) {
+    k_reduce_partials<<<passes, 256, 0, s>>>(part, rpart, warps, stride, diag, stage);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_march_forward(int Q, int coll, int storage, const MarchFwdArgs& g0, cudaStream_t s) {

@@ -1154,10 +1154,7 @@ FwdArgs fwd_args(lbm_handle& h) {
     a.mask = h.mask.as<uint32_t>();
     a.alpha = h.alpha.as<float>();
     a.ports = ports_at(h, h.t);
-    a.red = reduce_of(h);
     a.err = h.errflag.as<int>();
-    // the fused response sums reduce through the upper half of the scratch
-    a.red2 = Reduce{h.partial.as<double>() + (size_t)h.sms * 32 * 8, h.counter.as<unsigned>() + 1};
     a.phi = h.phi.as<float>();
     a.sp.vel = (float)(h.dx / h.dt);
     a.sp.dens = (float)h.density;
@@ -1175,35 +1172,61 @@ int coll_kernel(const lbm_handle& h) {
     return (h.P.n_proj == 1 && h.bulk_only) ? CK_MRT_BULK : CK_MRT;
 }
 
-// One step of the current state; diag / record / the current state's
-// response sums (16 doubles) optional.
-void step(lbm_handle& h, StepDiag* diag, float* record, bool record_s = false, double* stage = nullptr) {
+// One pass of the staged kernels over the current state: a step, or (collide
+// = false) load-only; the warps' partials of its admission record and
+// response sums and its record are optional.
+void pass(lbm_handle& h, bool collide, StepPartial* partial, double* rpartial, float* record, bool record_s,
+          uint32_t* warps) {
     FwdArgs a = fwd_args(h);
-    a.stage = stage;
+    if (!collide) a.dst = nullptr;
     a.apply_ports = h.pending ? 1 : 0;
-    a.diag = diag;
+    a.partial = partial;
+    a.rpartial = rpartial;
     a.record = record;
     a.record_s = record_s ? 1 : 0;
-    a.collide = 1;
+    a.collide = collide ? 1 : 0;
     a.step = (uint32_t)h.t;
-    CK(launch_forward(h.Q, coll_kernel(h), h.storage, a, grid_for(h), h.stream));
+    CK(launch_forward(h.Q, coll_kernel(h), h.storage, a, h.stream, warps));
+    if (!collide) return;
     h.cur ^= 1;
     h.restored = nullptr;
     h.pending = h.n_ports > 0;
     ++h.t;
 }
 
+// `passes` passes launched one by one; with inspect_last the last one is
+// load-only.  diag / record / stage point at the first pass's slots (stage: 16
+// doubles per pass).  The partials of up to 16 passes are combined at once.
+void staged_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* diag, float* record,
+                   int64_t record_stride, bool record_s, double* stage) {
+    const int64_t W = pass_warps(h.n(), h.sms), chunk = std::min<int64_t>(16, passes);
+    DevBuf buf;
+    if (diag || stage)
+        buf.alloc_pooled((size_t)(chunk * W) * (sizeof(StepPartial) + 64), &h.device_bytes, h.device, h.stream);
+    StepPartial* const part = buf.as<StepPartial>();
+    double* const rpart = buf.p ? reinterpret_cast<double*>(part + chunk * W) : nullptr;
+    for (int64_t i = 0; i < passes;) {
+        const int64_t k = std::min(chunk, passes - i);
+        uint32_t warps = 0;
+        for (int64_t j = 0; j < k; ++j)
+            pass(h, !(inspect_last && i + j == passes - 1), diag ? part + j * W : nullptr,
+                 stage ? rpart + j * W * 8 : nullptr, record ? record + (size_t)(i + j) * record_stride : nullptr,
+                 record_s, &warps);
+        if (diag || stage)
+            CK(launch_reduce_partials(part, rpart, warps, (uint32_t)W, (int)k, diag ? diag + i : nullptr,
+                                      stage ? stage + i * 16 : nullptr, h.stream));
+        i += k;
+    }
+}
+
+// One step of the current state.
+void step(lbm_handle& h, StepDiag* diag, float* record, bool record_s = false) {
+    staged_passes(h, 1, false, diag, record, 0, record_s, nullptr);
+}
+
 // Load-only pass of the current state (admission reductions and/or record).
-void inspect(lbm_handle& h, StepDiag* diag, float* record, bool record_s = false, double* stage = nullptr) {
-    FwdArgs a = fwd_args(h);
-    a.stage = stage;
-    a.dst = nullptr;
-    a.apply_ports = h.pending ? 1 : 0;
-    a.diag = diag;
-    a.record = record;
-    a.record_s = record_s ? 1 : 0;
-    a.collide = 0;
-    CK(launch_forward(h.Q, coll_kernel(h), h.storage, a, grid_for(h), h.stream));
+void inspect(lbm_handle& h, StepDiag* diag, float* record, bool record_s = false) {
+    staged_passes(h, 1, true, diag, record, 0, record_s, nullptr);
 }
 
 // A run of passes in one cooperative launch (lbm_march.cu) where the grid is
@@ -1238,13 +1261,7 @@ int64_t march_chunk(lbm_handle& h, bool stage) {
 void run_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* diag, float* record, int64_t record_stride,
                 bool record_s, double* stage) {
     if (passes < 3 || !marches(h, false)) {
-        for (int64_t i = 0; i < passes; ++i) {
-            StepDiag* d = diag ? diag + i : nullptr;
-            float* r = record ? record + (size_t)i * record_stride : nullptr;
-            double* st = stage ? stage + i * 16 : nullptr;
-            if (inspect_last && i == passes - 1) inspect(h, d, r, record_s, st);
-            else step(h, d, r, record_s, st);
-        }
+        staged_passes(h, passes, inspect_last, diag, record, record_stride, record_s, stage);
         return;
     }
     ensure_port_maps(h, h.t + passes);
@@ -1260,7 +1277,7 @@ void run_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* diag
         g.a.apply_ports = h.pending ? 1 : 0;
         g.a.record = record ? record + (size_t)i * record_stride : nullptr;
         g.a.record_s = record_s ? 1 : 0;
-        g.a.stage = stage ? stage + i * 16 : nullptr;
+        g.stage = stage ? stage + i * 16 : nullptr;
         g.a.step = (uint32_t)h.t;
         g.dst1 = h.pop_array(h.cur) + pop_pad(h.G) * storage_bytes(h.storage);
         g.n_pass = (int32_t)k;
@@ -1628,7 +1645,7 @@ void adjoint_step(lbm_handle& h, AdjState& st, const float* rec, bool want_norm,
     a.out_scale = st.target;
     a.abar_factor = st.s0;
     a.norm2 = want_norm ? h.norm2.as<double>() : nullptr;
-    CK(launch_adjoint(h.Q, coll_kernel(h), h.lam_storage, a, grid_for(h), h.stream));
+    CK(launch_adjoint(h.Q, coll_kernel(h), h.lam_storage, a, h.stream));
     h.lcur ^= 1;
     nee_move(h, h.lamA(), h.lam_storage);
     st.scale = st.target;
@@ -2708,7 +2725,7 @@ lbm_status step_vjp_impl(lbm_handle* h, const double* state, const double* lambd
     a.in_scale_inv = 1.f;
     a.out_scale = 1.f;
     a.abar_factor = 1.f;
-    CK(launch_adjoint(Q, coll_kernel(*h), LBM_STORE_F32, a, grid_for(*h), h->stream));
+    CK(launch_adjoint(Q, coll_kernel(*h), LBM_STORE_F32, a, h->stream));
     h->lcur ^= 1;
     check_errflag(*h);
     CK(launch_canon_lam(Q, LBM_STORE_F32, h->G, h->lamA(), h->mask.as<uint32_t>(), 1.f, h->scratch.as<float>(),
