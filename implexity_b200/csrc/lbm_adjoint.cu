@@ -37,7 +37,7 @@ struct AdjStage {
 // alpha cotangent ab_prev): the general path.
 template <int Q, int COLL, typename T, int AL, int STG, typename S>
 __device__ __forceinline__ void adj_one_cell(const AdjArgs& a, const S* st, int c, uint32_t x, uint32_t m, float ab_prev,
-                                             const T* B, T* D, uint32_t n, float s_in, float k_out, double& nsum) {
+                                             bool zwall, bool zlow, const T (&own)[ZWall<Q>::N], const T* B, T* D, uint32_t n, float s_in, float k_out, double& nsum) {
     const bool fluid = !(m & MASK_SOLID);
     if (!fluid) return;
     float v[Q];
@@ -45,11 +45,21 @@ __device__ __forceinline__ void adj_one_cell(const AdjArgs& a, const S* st, int 
 #pragma unroll
         for (int q = 0; q < Q; ++q)
             v[q] = Cvt<T>::to(st->run[q][(AL ? rund_aligned<Q, T, 1>(q) : a.rund[q]) + c]);
-        if (m & LINK_BITS) {
-            // transposed bounce-back: the cell's own opposite slot
+        // transposed bounce-back: the cell's own opposite slot
+        uint32_t links = m & LINK_BITS;
+        using Z = ZWall<Q>;
+        if (zwall) {  // (folded away where the step does not prefetch)
+#pragma unroll
+            for (int i = 0; i < Z::N; ++i) {
+                if (zlow) v[opp<Q>(Z::up(i))] = Cvt<T>::to(own[i]);
+                else v[Z::up(i)] = Cvt<T>::to(own[i]);
+            }
+            links &= ~(zlow ? Z::up_bits() : Z::down_bits());
+        }
+        if (links) {
 #pragma unroll
             for (int q = 1; q < Q; ++q)
-                if ((m >> opp<Q>(q)) & 1u) v[q] = Cvt<T>::to(B[opp<Q>(q) * n + x]);
+                if ((links >> opp<Q>(q)) & 1u) v[q] = Cvt<T>::to(B[opp<Q>(q) * n + x]);
         }
     } else {
 #pragma unroll
@@ -171,14 +181,28 @@ __global__ void __launch_bounds__(TPB, (sizeof(T) == 2 && Q == 19 ? 3 : 2)) k_ad
         uint32_t round = 0;
         const float s_in = 1.f / a.in_scale_inv;        // stored scale of the input
         const float k_out = a.out_scale * a.in_scale_inv;  // stored input -> stored output
-        for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        using Z = ZWall<Q>;
+        // FP16 256x128x128: 106.0 -> 101.9 us per step.  FP32 storage is bound by
+        // bandwidth and gains nothing (D3Q27 lost 10% to the registers), nor does
+        // the forward step, whose registers then spill (124 -> 135 us).
+        constexpr bool PREFETCH = sizeof(T) == 2;
+        ZWalk z(a.G, blockIdx.x * TILE + c0, gridDim.x * TILE);
+        for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, z.next()) {
             const uint32_t x = tile * TILE + c0;
+            // a z-wall cell's bounced cotangents, ahead of the tile
+            const bool zlow = PREFETCH && z.low(), zwall = PREFETCH && (zlow || z.high());
+            T own[Z::N];
+            if (zwall && x < n) {
+#pragma unroll
+                for (int i = 0; i < Z::N; ++i) own[i] = B[(zlow ? Z::up(i) : opp<Q>(Z::up(i))) * n + x];
+            }
             // the running alpha cotangent, read before the wait so that its
             // latency hides behind the staged copies and the collision
             const float ab_prev = (!a.overwrite_abar && x < n) ? a.abar[x] : 0.f;
             const bool ok = mbar_wait(&full[s], round & 1u, a.err);
             const S* st = stage_at<S>(smem, s);
-            adj_one_cell<Q, COLL, T, AL, STG>(a, st, c0, x, ok && x < n ? st->mask[c0] : MASK_SOLID, ab_prev, B, D, n,
+            adj_one_cell<Q, COLL, T, AL, STG>(a, st, c0, x, ok && x < n ? st->mask[c0] : MASK_SOLID, ab_prev, zwall,
+                                              zlow, own, B, D, n,
                                               s_in, k_out, nsum);
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[s]);

@@ -1620,6 +1620,55 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
     return r;
 }
 
+// ------------------------------------------------------------------ z walls
+// Axis 2 is the contiguous one, so a closed face across it has two cells in
+// every row of nz: at nz = 128 every other warp of the stepping kernels holds
+// a wall cell, and its bounce-back loads (the cell's own opposite slots) stall
+// the whole warp for a trip to L2.  Which populations those are follows from
+// the cell's coordinate alone, so the consumers load them before they wait for
+// the tile: the 5 (9) directions with c_z = +1 at the lower face, those with
+// c_z = -1 at the upper one.
+template <int Q>
+struct ZWall {
+    using L = Lat<Q>;
+    static constexpr int N = Q == 19 ? 5 : 9;
+    // the i-th direction with c_z = +1; the set of them as link bits
+    LBM_HD static constexpr int up(int i) {
+        int k = 0;
+        for (int q = 0; q < Q; ++q)
+            if (L::cz(q) == 1 && k++ == i) return q;
+        return 0;
+    }
+    LBM_HD static constexpr uint32_t up_bits() {
+        uint32_t b = 0;
+        for (int i = 0; i < N; ++i) b |= 1u << up(i);
+        return b;
+    }
+    LBM_HD static constexpr uint32_t down_bits() {
+        uint32_t b = 0;
+        for (int i = 0; i < N; ++i) b |= 1u << opp<Q>(up(i));
+        return b;
+    }
+};
+
+// The z coordinate of a thread's cell from tile to tile.
+struct ZWalk {
+    uint32_t k, step, nz;
+    bool closed;
+    __device__ __forceinline__ ZWalk(const Geometry& G, uint32_t x, uint32_t stride) {
+        nz = (uint32_t)G.nz;
+        k = x % nz;
+        step = stride % nz;
+        closed = !(G.periodic & 4);
+    }
+    __device__ __forceinline__ bool low() const { return closed && k == 0; }
+    __device__ __forceinline__ bool high() const { return closed && k == nz - 1; }
+    __device__ __forceinline__ void next() {
+        k += step;
+        if (k >= nz) k -= nz;
+    }
+};
+
 // Minimum population f = w + g (or w (1 + g/w) in 16-bit storage units) of
 // one cell: the minimum is taken per weight class (|c|^2) first.
 template <int Q, int SC>
