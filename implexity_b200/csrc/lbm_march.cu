@@ -37,13 +37,15 @@ namespace {
 constexpr int MT = 256;  // threads per block (128 where a grid then still fits one block per SM)
 
 // Neighbour offsets of one cell along each axis; a cell on a periodic face
-// (MASK_WRAP) gets the wrapped ones.
+// (MASK_WRAP) gets the wrapped ones.  Grids without periodic axes (WRAP = 0)
+// have the same offsets in every cell: they stay in uniform registers.
 struct Deltas {
     int32_t xm, xp, ym, yp, zm, zp;
 };
+template <int WRAP>
 __device__ __forceinline__ Deltas deltas_of(const Geometry& G, uint32_t x, uint32_t m) {
     Deltas d{-(int32_t)G.sx, (int32_t)G.sx, -(int32_t)G.sy, (int32_t)G.sy, -1, 1};
-    if (m & MASK_WRAP) {
+    if (WRAP && (m & MASK_WRAP)) {
         const uint32_t ij = x / (uint32_t)G.nz, k = x - ij * (uint32_t)G.nz;
         const uint32_t i = ij / (uint32_t)G.ny, j = ij - i * (uint32_t)G.ny;
         if (i == 0) d.xm += (int32_t)G.n;
@@ -112,8 +114,8 @@ __device__ __forceinline__ void copy_ports(PortMap* to, const PortMap* from, int
 }
 
 // ------------------------------------------------------------------ forward
-template <int Q, int COLL, typename T, int RSP, int DP>
-__global__ void __launch_bounds__(MT, (Q == 19 && !DP && !RSP ? 3 : 2)) k_march_forward(const __grid_constant__ MarchFwdArgs g) {
+template <int Q, int COLL, typename T, int RSP, int DP, int WRAP, int MB>
+__global__ void __launch_bounds__(MT, MB) k_march_forward(const __grid_constant__ MarchFwdArgs g) {
     using L = Lat<Q>;
     constexpr int SC = Cvt<T>::scaled ? 1 : 0;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -128,7 +130,7 @@ __global__ void __launch_bounds__(MT, (Q == 19 && !DP && !RSP ? 3 : 2)) k_march_
     __syncthreads();
     uint32_t m = 0;
     float alpha = 0.f;
-    Deltas dl{};
+    Deltas dl = deltas_of<0>(a.G, 0, 0);
     for (int pass = 0; pass < g.n_pass; ++pass) {
         const T* A = static_cast<const T*>(pass == 0 ? a.src : (pass & 1) ? a.dst : g.dst1);
         T* D = static_cast<T*>((pass & 1) ? g.dst1 : a.dst);
@@ -142,7 +144,7 @@ __global__ void __launch_bounds__(MT, (Q == 19 && !DP && !RSP ? 3 : 2)) k_march_
             if (!single || pass == 0) {
                 m = a.mask[x];
                 alpha = a.alpha[x];
-                dl = deltas_of(a.G, x, m);
+                if (WRAP) dl = deltas_of<WRAP>(a.G, x, m);
             }
             if (m & MASK_SOLID) {
                 if constexpr (RSP) rsum[5] += (double)a.phi[x];
@@ -241,8 +243,8 @@ __global__ void __launch_bounds__(MT, (Q == 19 && !DP && !RSP ? 3 : 2)) k_march_
 // ------------------------------------------------------------------ adjoint
 // A run of transposed steps (adj_one_cell of lbm_adjoint.cu, pass by pass):
 // pass i is linearised at the record i slots before a.record.
-template <int Q, int COLL, typename T, int STG>
-__global__ void __launch_bounds__(MT, (Q == 19 && !STG ? 3 : 2)) k_march_adjoint(const __grid_constant__ MarchAdjArgs g) {
+template <int Q, int COLL, typename T, int STG, int WRAP, int MB>
+__global__ void __launch_bounds__(MT, MB) k_march_adjoint(const __grid_constant__ MarchAdjArgs g) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int go;
     PortMap* ports = reinterpret_cast<PortMap*>(smem);
@@ -255,7 +257,7 @@ __global__ void __launch_bounds__(MT, (Q == 19 && !STG ? 3 : 2)) k_march_adjoint
     double nsum = 0.0;
     uint32_t m = 0;
     float alpha = 0.f, ab_run = 0.f;
-    Deltas dl{};
+    Deltas dl = deltas_of<0>(a.G, 0, 0);
     for (int pass = 0; pass < g.n_pass; ++pass) {
         const T* B = static_cast<const T*>((pass & 1) ? a.dst : a.src);
         T* D = static_cast<T*>((pass & 1) ? const_cast<void*>(a.src) : a.dst);
@@ -268,7 +270,7 @@ __global__ void __launch_bounds__(MT, (Q == 19 && !STG ? 3 : 2)) k_march_adjoint
             if (!single || pass == 0) {
                 m = a.mask[x];
                 alpha = a.alpha[x];
-                dl = deltas_of(a.G, x, m);
+                if (WRAP) dl = deltas_of<WRAP>(a.G, x, m);
                 ab_run = (m & MASK_SOLID) || (a.overwrite_abar && pass == 0) ? 0.f : a.abar[x];
             }
             if (m & MASK_SOLID) continue;
@@ -336,6 +338,21 @@ __global__ void __launch_bounds__(MT, (Q == 19 && !STG ? 3 : 2)) k_march_adjoint
 // ------------------------------------------------------------------ launch
 constexpr size_t PORT_SMEM = MAX_PORTS * sizeof(PortMap);
 
+// Blocks per SM: two leave a thread 128 registers (no spills), three 80 (36 to
+// 120 bytes spilled in D3Q19) but half as many threads again.  One round over
+// the resident threads takes about 1.4 times as long with three, so they pay
+// where they save enough rounds: us per FP32 forward step with two / three,
+// 110 592 cells (2 rounds / 1) 5.8 / 5.3, 139 776 (2 / 2) 6.0 / 7.1, 262 144
+// (4 / 3) 9.8 / 10.5, 614 400 (9 / 6) 24.2 / 21.5, 1 032 192 (14 / 10) 41.6 /
+// 39.0; the adjoint alike.
+inline bool three_blocks(int64_t n) {
+    int sms = 148, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t two = (n + 2 * MT * sms - 1) / (2 * MT * sms), three = (n + 3 * MT * sms - 1) / (3 * MT * sms);
+    return 7 * three < 5 * two;
+}
+
 struct MarchShape {
     int grid, threads;
 };
@@ -363,7 +380,10 @@ cudaError_t launch_cooperative(K kernel, const MarchShape& s, A& args, cudaStrea
 
 template <int Q, int COLL, typename T, int RSP, int DP>
 cudaError_t run_march(MarchFwdArgs& g, cudaStream_t s) {
-    const auto kernel = k_march_forward<Q, COLL, T, RSP, DP>;
+    void (*kernel)(const MarchFwdArgs) =
+        g.a.G.periodic ? k_march_forward<Q, COLL, T, RSP, DP, 1, 2> : k_march_forward<Q, COLL, T, RSP, DP, 0, 2>;
+    if constexpr (Q == 19 && !RSP && !DP)
+        if (!g.a.G.periodic && three_blocks(g.a.G.n)) kernel = k_march_forward<Q, COLL, T, RSP, DP, 0, 3>;
     const MarchShape sh = march_shape(kernel, g.a.G.n);
     const uint32_t warps = (uint32_t)(sh.grid * sh.threads / 32);
     const int64_t per_pass = (int64_t)warps * ((g.diag ? sizeof(StepPartial) : 0) + (RSP ? 64 : 0));
@@ -390,11 +410,12 @@ cudaError_t run_march_forward(MarchFwdArgs& g, cudaStream_t s) {
 
 template <int Q, int COLL, typename T>
 cudaError_t run_march_adjoint(MarchAdjArgs& g, cudaStream_t s) {
-    if (g.a.rec_planes == 10) {
-        const auto kernel = k_march_adjoint<Q, COLL, T, 1>;
-        return launch_cooperative(kernel, march_shape(kernel, g.a.G.n), g, s);
-    }
-    const auto kernel = k_march_adjoint<Q, COLL, T, 0>;
+    void (*kernel)(const MarchAdjArgs) =
+        g.a.rec_planes == 10
+            ? (g.a.G.periodic ? k_march_adjoint<Q, COLL, T, 1, 1, 2> : k_march_adjoint<Q, COLL, T, 1, 0, 2>)
+            : (g.a.G.periodic ? k_march_adjoint<Q, COLL, T, 0, 1, 2> : k_march_adjoint<Q, COLL, T, 0, 0, 2>);
+    if constexpr (Q == 19)
+        if (g.a.rec_planes != 10 && !g.a.G.periodic && three_blocks(g.a.G.n)) kernel = k_march_adjoint<Q, COLL, T, 0, 0, 3>;
     return launch_cooperative(kernel, march_shape(kernel, g.a.G.n), g, s);
 }
 

@@ -1234,18 +1234,27 @@ void inspect(lbm_handle& h, StepDiag* diag, float* record, bool record_s = false
 // extrapolating ports (a second kernel moves their cotangents after every
 // step), the general MRT collision or x-slabs (halos).
 // The limits, us per step of the staged kernels / of a run (B200):
-//   cells                  27 648      262 144      614 400     1 032 192    2 097 152
-//   forward FP32       12.4 / 3.5  18.5 / 11.2  27.8 / 23.5  43.3 / 41.3  67.9 / 73.5
-//   forward FP16       14.4 / 3.5  19.5 / 11.1  25.5 / 18.7  37.1 / 32.1  62.5 / 60.2
-//   forward D3Q27      16.5 / 4.4  24.7 / 12.4  45.7 / 33.2  58.0 / 51.0   101 / 98
-//   forward FP64 coll. 16.2 / 4.8  27.0 / 15.3  44.8 / 34.9  71.9 / 55.6   116 / 107
-//   adjoint FP32        8.3 / 3.4  14.0 / 11.1  25.9 / 28.4  38.8 / 49.7
-//   adjoint FP16        8.3 / 3.3  12.5 / 10.7  20.6 / 18.6  32.8 / 37.2
-//   adjoint D3Q27      10.4 / 4.2  18.5 / 12.5  41.5 / 35.6  54.0 / 54.7
-// (FP64 collision at 4 194 304 cells: 224 / 216.)
-bool marches(const lbm_handle& h, bool adjoint) {
-    const int64_t most = adjoint ? (h.Q == 19 && h.lam_storage == LBM_STORE_F32 ? 400 << 10 : 640 << 10)
-                                 : (h.collision_fp64 ? 4 << 20 : 1 << 20);
+//   cells                       27 648      262 144      614 400      805 376    1 032 192   2 097 152   4 194 304
+//   forward FP32            8.7 / 3.4   12.9 / 9.4  23.1 / 21.4  29.6 / 33.0
+//   forward FP16            9.6 / 3.4   14.9 / 9.7  21.1 / 18.0  27.4 / 22.0  33.6 / 29.1  59.6 / 57.0   114 / 108
+//   forward D3Q27 FP32     12.7 / 4.5  19.3 / 12.9  40.5 / 35.3  44.0 / 43.1  53.7 / 53.7  95.5 / 103
+//   forward D3Q27 FP16     13.2 / 4.5  21.0 / 12.7  37.5 / 24.7  43.3 / 32.2  52.0 / 41.8  96.6 / 79.8   182 / 151
+//   forward FP64 collision 12.3 / 4.7  21.6 / 14.9  39.5 / 35.0  52.5 / 45.1  66.0 / 56.5   110 / 107
+//   adjoint FP32            8.3 / 3.1   14.2 / 9.0  24.9 / 23.9  30.6 / 33.7
+//   adjoint FP16            8.3 / 3.2   12.4 / 9.2  20.6 / 17.4  24.7 / 21.9  32.5 / 35.5
+//   adjoint D3Q27          10.3 / 4.0  18.5 / 12.2  40.1 / 34.6  43.8 / 42.6  54.1 / 53.3  99.2 / 103
+// and with the response sums 20.0 / 15.4 (262 144, FP32), 33.7 / 36.3 (614 400),
+// D3Q27 53.4 / 45.9 and 68.0 / 67.7 (1 032 192); with the stage seeds (a dozen
+// divisions per cell then) 24.0 / 22.9 and 47.4 / 52.6, D3Q27 30.2 / 26.2 and
+// 58.2 / 61.6.  The direct loads of a run
+// cost a 16-bit step less than the staged ring does, at every size measured.
+bool marches(const lbm_handle& h, bool adjoint, bool stage) {
+    const bool wide = (adjoint ? h.lam_storage : h.storage) == LBM_STORE_F32, q27 = h.Q == 27;
+    int64_t most;
+    if (adjoint) most = stage ? 400 << 10 : q27 ? 1 << 20 : wide ? 640 << 10 : 900 << 10;
+    else if (!wide) most = stage && !q27 ? 1 << 20 : 4 << 20;
+    else if (h.collision_fp64) most = 2 << 20;
+    else most = q27 ? 900 << 10 : stage ? 400 << 10 : 640 << 10;
     return h.cooperative && h.n() <= most && coll_kernel(h) != CK_MRT && h.nee_groups.empty() && !h.slab;
 }
 
@@ -1260,7 +1269,7 @@ int64_t march_chunk(lbm_handle& h, bool stage) {
 // point at the first pass's slots (record_stride floats, 16 doubles apart).
 void run_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* diag, float* record, int64_t record_stride,
                 bool record_s, double* stage) {
-    if (passes < 3 || !marches(h, false)) {
+    if (passes < 3 || !marches(h, false, stage != nullptr)) {
         staged_passes(h, passes, inspect_last, diag, record, record_stride, record_s, stage);
         return;
     }
@@ -1659,7 +1668,7 @@ void adjoint_step(lbm_handle& h, AdjState& st, const float* rec, bool want_norm,
 // asked for.
 void adjoint_run(lbm_handle& h, AdjState& st, const float* rec, int64_t stride, int64_t count, bool want_norm, int64_t t,
                  const SeedParams* stage = nullptr, int64_t stage_steps = 0, int rec_planes = 4) {
-    if (count < 2 || !marches(h, true)) {
+    if (count < 2 || !marches(h, true, stage != nullptr)) {
         for (int64_t i = 0; i < count; ++i)
             adjoint_step(h, st, rec - i * stride, want_norm && i == count - 1, stride ? t - i : t,
                          i < stage_steps ? stage : nullptr, rec_planes);
@@ -1946,16 +1955,10 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
         // the transposed steps of states [s0, e0) in reverse; their records
         // follow each other from first_rec on
         auto transposed_span = [&](const float* first_rec, int64_t s0, int64_t e0, int64_t seg_start) {
-            CK(cudaEventRecord(ea0, h.stream));
             // (state 0 is not part of the average)
             adjoint_run(h, st, first_rec + (size_t)(e0 - 1 - s0) * rec_stride, (int64_t)rec_stride, e0 - s0,
                         s0 == seg_start, e0 - 1, stage ? &sp : nullptr, stage ? e0 - std::max<int64_t>(s0, 1) : 0,
                         rec_planes);
-            CK(cudaEventRecord(ea1, h.stream));
-            CK(cudaEventSynchronize(ea1));
-            float a2 = 0;
-            CK(cudaEventElapsedTime(&a2, ea0, ea1));
-            ms_adj += a2;
         };
         // records of states [s0, e0), then their transposed steps in reverse
         auto reverse_span = [&](int64_t s0, int64_t e0, int64_t seg_start) {
@@ -1964,19 +1967,32 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
             recomputed += e0 - s0 - 1;
             CK(cudaEventRecord(ef1, h.stream));
             transposed_span(rec, s0, e0, seg_start);
-            float a1 = 0;
+            CK(cudaEventRecord(ea1, h.stream));
+            CK(cudaEventSynchronize(ea1));
+            float a1 = 0, a2 = 0;
             CK(cudaEventElapsedTime(&a1, ef0, ef1));
+            CK(cudaEventElapsedTime(&a2, ef1, ea1));
             ms_fwd += a1;
+            ms_adj += a2;
         };
         auto restore = [&](const Checkpoint& c) {
             CK(cudaMemcpyAsync(h.pop_array(h.cur), c.buf->p, c.buf->bytes, cudaMemcpyDeviceToDevice, h.stream));
             h.pending = c.pending;
             h.t = c.t;
         };
-        for (int64_t s0 = whole.p ? (T - 1) / K * K : -1; s0 >= 0; s0 -= K) {
-            transposed_span(rec + (size_t)s0 * rec_stride, s0, std::min(s0 + K, T), s0);
-            // rescale the stored adjoint at segment boundaries
-            st.target = next_scale(h, read_norm(h) / st.scale, st.scale);
+        if (whole.p) {
+            // a power of two does not change an FP32 cotangent: it is rescaled
+            // only to stay in range, every few segments, where a 16-bit one is
+            // at every segment's end
+            const int64_t span = o.lambda_storage == LBM_STORE_F32 ? std::max<int64_t>(K, 256) : K;
+            CK(cudaEventRecord(ea0, h.stream));
+            for (int64_t s0 = (T - 1) / span * span; s0 >= 0; s0 -= span) {
+                transposed_span(rec + (size_t)s0 * rec_stride, s0, std::min(s0 + span, T), s0);
+                st.target = next_scale(h, read_norm(h) / st.scale, st.scale);
+            }
+            CK(cudaEventRecord(ea1, h.stream));
+            CK(cudaEventSynchronize(ea1));
+            CK(cudaEventElapsedTime(&ms_adj, ea0, ea1));
         }
         for (int64_t ci = (int64_t)h.ckpts.size() - 1; ci >= 0; --ci) {
             Checkpoint& c = h.ckpts[ci];
