@@ -1165,9 +1165,9 @@ __device__ __forceinline__ float response_vjp(float rp, const float (&u)[3], con
                                               float dpw, bool port, const SeedParams& sp, const Physics& P,
                                               float (&fb)[Q]) {
     using L = Lat<Q>;
-    const float k = 1.f - 0.5f / sp.tau;
-    const float nu = (sp.tau - 0.5f) / 3.f;
+    const float k = sp.visc_k;
     const float rho = 1.f + rp;
+    const float ir = 1.f / rho;
     float F[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) F[d] = rho * (P.a[d] - alpha * u[d]);
@@ -1176,7 +1176,7 @@ __device__ __forceinline__ float response_vjp(float rp, const float (&u)[3], con
     float ss = 0.f;
 #pragma unroll
     for (int e = 0; e < 6; ++e) {
-        const float pi = S[e] - (e < 3 ? rp / 3.f : 0.f) - rho * u[ia[e]] * u[ib[e]];
+        const float pi = S[e] - (e < 3 ? rp * (1.f / 3.f) : 0.f) - rho * u[ia[e]] * u[ib[e]];
         const float t = 0.5f * (u[ia[e]] * F[ib[e]] + u[ib[e]] * F[ia[e]]);
         sig[e] = -k * (pi + t);
         ss += (e < 3 ? 1.f : 2.f) * sig[e] * sig[e];
@@ -1188,18 +1188,19 @@ __device__ __forceinline__ float response_vjp(float rp, const float (&u)[3], con
     const float R = rho * sp.dens;
     const float W3 = sp.w[3], W4 = sp.w[4], W7 = sp.w[7];
     float rb = 0.f, abar = 0.f, ub[3], Fb[3] = {0.f, 0.f, 0.f}, Sb[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const float kin = W3 + W4 * alpha / sp.dt_s;
+    const float kin = W3 + W4 * alpha * sp.inv_dt;
 #pragma unroll
     for (int d = 0; d < 3; ++d) ub[d] = sp.w[d] * V + kin * R * 2.f * U[d] * V;
     rb += kin * sp.dens * usq;
-    abar += W4 * R / sp.dt_s * usq;
-    if (port) rb += sp.w[6] * dpw * sp.dens * V * V / 3.f;
+    abar += W4 * R * sp.inv_dt * usq;
+    if (port) rb += sp.w[6] * dpw * sp.dens * V * V * (1.f / 3.f);
     if (W7 != 0.f) {
-        rb += -W7 * ss / (2.f * rho * rho * nu);
+        const float wv = W7 * sp.inv_nu * ir, kw = -k * wv;
+        rb -= 0.5f * wv * ss * ir;
 #pragma unroll
         for (int e = 0; e < 6; ++e) {
             const float mult = (e < 3 ? 1.f : 2.f);  // off-diagonals appear twice
-            const float pb = -k * W7 * sig[e] / (rho * nu) * mult;
+            const float pb = kw * sig[e] * mult;
             const int i0 = ia[e], i1 = ib[e];
             Sb[e] += pb;
             rb -= pb * ((e < 3 ? 1.f / 3.f : 0.f) + u[i0] * u[i1]);
@@ -1224,13 +1225,13 @@ __device__ __forceinline__ float response_vjp(float rp, const float (&u)[3], con
         ub[d] -= Fb[d] * rho * alpha;
     }
     const float s = 1.f + 0.5f * alpha;
-    const float inv = 1.f / (s * rho);
+    const float inv_s = 1.f / s, inv = inv_s * ir;
     float mb[3], sbar = 0.f;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         mb[d] = ub[d] * inv;
         rb -= ub[d] * (s * u[d] - 0.5f * P.a[d]) * inv;
-        sbar -= ub[d] * u[d] / s;
+        sbar -= ub[d] * u[d] * inv_s;
     }
     abar += 0.5f * sbar;
 #pragma unroll
@@ -1256,8 +1257,7 @@ __device__ __forceinline__ float response_vjp(float rp, const float (&u)[3], con
 template <int Q>
 __device__ __forceinline__ void response_cell(float rp, const float (&u)[3], const float (&S)[6], float alpha,
                                               const SeedParams& sp, const Physics& P, float (&out)[6]) {
-    const float k = 1.f - 0.5f / sp.tau;
-    const float nu = (sp.tau - 0.5f) / 3.f;
+    const float k = sp.visc_k;
     const float rho = 1.f + rp;
     float F[3];
 #pragma unroll
@@ -1266,7 +1266,7 @@ __device__ __forceinline__ void response_cell(float rp, const float (&u)[3], con
     float ss = 0.f;
 #pragma unroll
     for (int e = 0; e < 6; ++e) {
-        const float pi = S[e] - (e < 3 ? rp / 3.f : 0.f) - rho * u[ia[e]] * u[ib[e]];
+        const float pi = S[e] - (e < 3 ? rp * (1.f / 3.f) : 0.f) - rho * u[ia[e]] * u[ib[e]];
         const float t = 0.5f * (u[ia[e]] * F[ib[e]] + u[ib[e]] * F[ia[e]]);
         const float sg = -k * (pi + t);
         ss += (e < 3 ? 1.f : 2.f) * sg * sg;
@@ -1279,8 +1279,8 @@ __device__ __forceinline__ void response_cell(float rp, const float (&u)[3], con
     out[1] = U[1];
     out[2] = U[2];
     out[3] = R * usq;
-    out[4] = R * alpha / sp.dt_s * usq;
-    out[5] = ss / (2.f * rho * nu);
+    out[4] = R * alpha * sp.inv_dt * usq;
+    out[5] = 0.5f * sp.inv_nu * ss / rho;
 }
 
 // ------------------------------------------------------------------ reductions

@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(BLOCK) k_objective(ObjArgs a) {
         sp.dens = a.dens;
         sp.dt_s = a.dt_s;
         sp.tau = a.tau;
+        set_viscous(sp);
         const float* u = M.u;
         {
             float fb[Q];

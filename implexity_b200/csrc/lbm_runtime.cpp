@@ -1160,6 +1160,7 @@ FwdArgs fwd_args(lbm_handle& h) {
     a.sp.dens = (float)h.density;
     a.sp.dt_s = (float)h.dt;
     a.sp.tau = (float)h.tau;
+    set_viscous(a.sp);
     a.dp_collision = h.collision_fp64 ? 1 : 0;
     a.omega_cell = h.tau_per_cell ? h.omega_cell.as<float>() : nullptr;
     return a;
@@ -1739,6 +1740,7 @@ SeedParams stage_seed(const lbm_handle& h, const double* w, double scale) {
     sp.dens = (float)h.density;
     sp.dt_s = (float)h.dt;
     sp.tau = (float)h.tau;
+    set_viscous(sp);
     return sp;
 }
 
