@@ -52,6 +52,19 @@ def adj_bytes(q, s_lam):
     return 16 + 4 + 2 * q * s_lam + 8
 
 
+def launches(cells, T, storage, iterations):
+    """Kernels launched by one design iteration (D3Q19): input narrowing, design map, two initial
+    states, the forward passes, responses, two seeds, the transposed steps (residual checked every
+    100) and two of the design-map transpose.  Staged forward passes are one launch each and one per
+    16 for their partials; runs of steps (16-bit storage, or a small grid) one for as many passes as
+    8 MB of partials hold (128 at most) and one for the partials."""
+    wide = storage == "float32"
+    run = min(128, max(8, (8 << 20) // (min(-(-cells // 256) * 8, 148 * 64) * 32)))
+    forward = T + 1 + -(-(T + 1) // 16) if wide and cells > 640 << 10 else 2 * -(-(T + 1) // run)
+    adjoint = iterations if cells > (640 << 10 if wide else 900 << 10) else iterations / 100
+    return 1 + 1 + 2 + forward + 1 + 2 + adjoint + 2
+
+
 def peaks():
     p = ROOT / "MEASURED_PEAKS.json"
     if p.exists():
@@ -233,7 +246,7 @@ def run_gpu(args, rank, world, local):
             "adjoint_roofline": adj_roof,
             "h2d_bytes_per_step": raw.size * 8,
             "d2h_bytes_per_step": raw.size * 8 + 8 * 8,
-            "launches_per_step": 1 + 1 + T + 1 + 1 + 2 + iters / args.steps + 2,
+            "launches_per_step": launches(cells, T, storage, iters / args.steps),
             "clocks": clk.summary(),
             "responses": [float(x) for x in r],
         }

@@ -10,6 +10,7 @@
 #include <charconv>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -397,11 +398,6 @@ struct DevBuf {
         pooled = nullptr;
         bytes = 0;
     }
-    // exactly b bytes (releases a larger buffer)
-    void fit(size_t b, int64_t* ctr) {
-        if (p && bytes != b) reset();
-        alloc(b, ctr);
-    }
     void alloc(size_t b, int64_t* ctr) {
         if (p && bytes >= b) return;
         reset();
@@ -432,6 +428,15 @@ struct DevBuf {
             p = nullptr;
         }
         alloc(b, ctr);
+    }
+    // at least b bytes of the pool: the buffers of a handle's first gradient or
+    // read-back, which a new handle then takes from an old one
+    void grow(size_t b, int64_t* ctr, int device, cudaStream_t s) {
+        if (!p || bytes < b) alloc_pooled(b, ctr, device, s);
+    }
+    // exactly b bytes of the pool (releases a larger buffer)
+    void fit(size_t b, int64_t* ctr, int device, cudaStream_t s) {
+        if (!p || bytes != b) alloc_pooled(b, ctr, device, s);
     }
     template <typename T>
     T* as() const {
@@ -468,6 +473,7 @@ void pin_handles(int by) {
 struct PinLease {
     void* p = nullptr;
     size_t bytes = 0;
+    bool pinned = true;  // false: the host would not lock more pages; the copies then go through the driver's
     explicit PinLease(size_t want) {
         size_t size = 64 << 10;
         while (size < want) size *= 2;
@@ -482,13 +488,22 @@ struct PinLease {
                     return;
                 }
         }
-        CK(cudaMallocHost(&p, size));
+        if (cudaMallocHost(&p, size) != cudaSuccess) {
+            cudaGetLastError();
+            p = std::malloc(size);
+            if (!p) throw std::bad_alloc();
+            pinned = false;
+        }
         bytes = size;
     }
     PinLease(const PinLease&) = delete;
     PinLease& operator=(const PinLease&) = delete;
     // (a lease ends after its call's last synchronisation: no copy is in flight)
     ~PinLease() {
+        if (!pinned) {
+            std::free(p);
+            return;
+        }
         PinList& L = pin_list();
         std::lock_guard<std::mutex> lock(L.mu);
         L.idle.emplace_back(p, bytes);
@@ -1265,6 +1280,18 @@ int64_t march_chunk(lbm_handle& h, bool stage) {
     return std::max<int64_t>(8, std::min<int64_t>(128, (8 << 20) / per));
 }
 
+// A run that does not fit the device as it is (another context holds part of
+// it) is not launched: the handle steps launch by launch from then on.
+bool launched(lbm_handle& h, cudaError_t e) {
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        h.cooperative = false;
+        return false;
+    }
+    CK(e);
+    return true;
+}
+
 // `passes` forward passes from the current state; with inspect_last the last
 // one is load-only (inspect), else every pass steps.  diag / record / stage
 // point at the first pass's slots (record_stride floats, 16 doubles apart).
@@ -1299,7 +1326,10 @@ void run_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* diag
         g.bar = reinterpret_cast<unsigned*>(h.word(2));
         g.scratch = partial.p;
         g.scratch_bytes = scratch;
-        CK(launch_march_forward(h.Q, coll_kernel(h), h.storage, g, h.stream));
+        if (!launched(h, launch_march_forward(h.Q, coll_kernel(h), h.storage, g, h.stream))) {
+            run_passes(h, passes - i, inspect_last, g.diag, g.a.record, record_stride, record_s, g.stage);
+            return;
+        }
         const int64_t steps = k - (inspects ? 1 : 0);
         if (steps > 0) {
             h.cur ^= (int)(steps & 1);
@@ -1391,7 +1421,9 @@ void check_errflag(lbm_handle& h) {
     CK(cudaStreamSynchronize(h.stream));
     if (e) {
         CK(cudaMemsetAsync(h.errflag.p, 0, sizeof(int), h.stream));
-        throw CudaError("a staged bulk copy did not complete within its bounded wait");
+        // blocks that gave up did not take their ticket of a sum
+        CK(cudaMemsetAsync(h.counter.p, 0, 2 * sizeof(unsigned), h.stream));
+        throw CudaError("a staged bulk copy or a barrier between steps did not complete within its bounded wait");
     }
 }
 
@@ -1408,11 +1440,11 @@ lbm_status run_admitted(lbm_handle& h, int64_t steps, lbm_diag_t* out, int64_t K
                         float* record = nullptr, int64_t record_stride = 0, bool record_s = false) {
     require_design(h);
     int64_t* ctr = &h.device_bytes;
-    h.diag.alloc((size_t)(steps + 1) * sizeof(StepDiag), ctr);
+    h.diag.grow((size_t)(steps + 1) * sizeof(StepDiag), ctr, h.device, h.stream);
     StepDiag* d = h.diag.as<StepDiag>();
     ensure_port_maps(h, h.t + steps);
     h.tavg_valid = false;
-    if (averages) h.tsums.alloc((size_t)(steps + 1) * 16 * sizeof(double), ctr);
+    if (averages) h.tsums.grow((size_t)(steps + 1) * 16 * sizeof(double), ctr, h.device, h.stream);
     CK(cudaEventRecord(h.ev0, h.stream));
     for (int64_t s = 0; s <= steps;) {
         if (K > 0 && s < steps && s % K == 0) {
@@ -1443,7 +1475,9 @@ lbm_status run_admitted(lbm_handle& h, int64_t steps, lbm_diag_t* out, int64_t K
     return admit(h, hd, out, ms);
 }
 
-void ensure_scratch(lbm_handle& h) { h.scratch.alloc((size_t)h.n() * h.Q * sizeof(float), &h.device_bytes); }
+void ensure_scratch(lbm_handle& h) {
+    h.scratch.grow((size_t)h.n() * h.Q * sizeof(float), &h.device_bytes, h.device, h.stream);
+}
 
 ObjArgs obj_args(lbm_handle& h) {
     ObjArgs a{};
@@ -1608,8 +1642,8 @@ int64_t plane_piece(int64_t n, int planes) { return std::min(n, PIN_CAP / (4 * p
 void design_transpose(lbm_handle& h, const float* phibar, const float* abar, float abar_scale,
                       const float* abar_final) {
     int64_t* ctr = &h.device_bytes;
-    h.scale.alloc((size_t)h.n() * 4, ctr);
-    h.grad.alloc((size_t)h.n() * 4, ctr);
+    h.scale.grow((size_t)h.n() * 4, ctr, h.device, h.stream);
+    h.grad.grow((size_t)h.n() * 4, ctr, h.device, h.stream);
     DesignArgs a = design_args(h);
     a.phibar = phibar;
     a.abar = abar;
@@ -1712,7 +1746,11 @@ void adjoint_run(lbm_handle& h, AdjState& st, const float* rec, int64_t stride, 
         g.port_stride = h.pulsatile && stride ? h.n_ports : 0;
         g.record_stride = stride;
         g.bar = reinterpret_cast<unsigned*>(h.word(2));
-        CK(launch_march_adjoint(h.Q, coll_kernel(h), h.lam_storage, g, h.stream));
+        if (!launched(h, launch_march_adjoint(h.Q, coll_kernel(h), h.lam_storage, g, h.stream))) {
+            adjoint_run(h, st, rec - i * stride, stride, count - i, want_norm, stride ? t - i : t, stage,
+                        std::max<int64_t>(0, stage_steps - i), rec_planes);
+            return;
+        }
         h.lcur ^= (int)(k & 1);
         st.scale = st.target;
         st.first = false;
@@ -1773,8 +1811,8 @@ float power_of_two(double v) {
 double seed(lbm_handle& h, const double* w, AdjState& st, float* record, double stage_scale = 1.0) {
     int64_t* ctr = &h.device_bytes;
     const int64_t n = h.n();
-    h.abar_final.alloc((size_t)n * 4, ctr);
-    h.phibar.alloc((size_t)n * 4, ctr);
+    h.abar_final.grow((size_t)n * 4, ctr, h.device, h.stream);
+    h.phibar.grow((size_t)n * 4, ctr, h.device, h.stream);
     h.norm2.alloc(2 * sizeof(double), ctr);
     ObjArgs a = obj_args(h);
     response_weights(h, w, stage_scale, a.w);
@@ -1807,8 +1845,8 @@ void alloc_adjoint(lbm_handle& h, int lam_storage) {
     const int64_t n = h.n();
     if (h.lam.p && h.lam_storage != lam_storage) h.lam.reset();
     h.lam_storage = lam_storage;
-    h.lam.alloc(2 * h.array_bytes(lam_storage), ctr);
-    h.abar.alloc((size_t)n * 4, ctr);
+    h.lam.grow(2 * h.array_bytes(lam_storage), ctr, h.device, h.stream);
+    h.abar.grow((size_t)n * 4, ctr, h.device, h.stream);
     h.norm2.alloc(2 * sizeof(double), ctr);
 }
 
@@ -1832,7 +1870,7 @@ lbm_status gradient_steady(lbm_handle& h, const double* w, const lbm_adjoint_opt
     if (!h.forward_done) throw StateError("lbm_forward must succeed before lbm_gradient");
     alloc_adjoint(h, o.lambda_storage);
     int64_t* ctr = &h.device_bytes;
-    h.record.alloc(((size_t)h.n() * 4 + CELL_PAD) * sizeof(float), ctr);
+    h.record.grow(((size_t)h.n() * 4 + CELL_PAD) * sizeof(float), ctr, h.device, h.stream);
     AdjState st;
     CK(cudaEventRecord(h.ev0, h.stream));
     const double n0 = seed(h, w, st, h.record.as<float>());
@@ -1949,7 +1987,7 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
         const int64_t spans = (K + fit - 1) / fit;
         KR = (K + spans - 1) / spans;
     }
-    if (!whole.p) h.record.fit(rec_bytes * (size_t)KR + CELL_PAD * sizeof(float), ctr);
+    if (!whole.p) h.record.fit(rec_bytes * (size_t)KR + CELL_PAD * sizeof(float), ctr, h.device, h.stream);
     h.ckpts.clear();
     // forward with checkpoints, then admission (the reference re-runs parts())
     init_state(h);
@@ -2114,7 +2152,7 @@ lbm_status gradient_binomial(lbm_handle& h, const double* w, const lbm_adjoint_o
     const int rec_planes = stage ? 10 : 4;
     alloc_adjoint(h, o.lambda_storage);
     int64_t* ctr = &h.device_bytes;
-    h.record.fit((size_t)h.n() * rec_planes * sizeof(float) + CELL_PAD * sizeof(float), ctr);
+    h.record.fit((size_t)h.n() * rec_planes * sizeof(float) + CELL_PAD * sizeof(float), ctr, h.device, h.stream);
     const size_t ab = h.array_bytes(h.storage);
     std::vector<Checkpoint> slots((size_t)o.snapshots);
     // a restored slot stands for the current state only while the slots live
@@ -2139,7 +2177,7 @@ lbm_status gradient_binomial(lbm_handle& h, const double* w, const lbm_adjoint_o
     };
     // forward sweep with the admission record of every state
     init_state(h);
-    h.diag.alloc((size_t)(T + 1) * sizeof(StepDiag), ctr);
+    h.diag.grow((size_t)(T + 1) * sizeof(StepDiag), ctr, h.device, h.stream);
     StepDiag* d = h.diag.as<StepDiag>();
     ensure_port_maps(h, T);
     bool prev_pending = false;
@@ -2352,6 +2390,10 @@ void lbm_destroy(lbm_handle* h) {
     h->slab_adj = nullptr;
     if (h->stream) cudaStreamSynchronize(h->stream);
     h->ckpts.clear();
+    // the pool's buffers go back in the order of the stream, before it goes
+    for (DevBuf* b : {&h->lam, &h->record, &h->abar, &h->abar_final, &h->phibar, &h->scale, &h->grad, &h->scratch, &h->diag,
+                      &h->tsums})
+        b->reset();
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -2723,7 +2765,7 @@ lbm_status step_vjp_impl(lbm_handle* h, const double* state, const double* lambd
         h->tau_bar.alloc((size_t)N * sizeof(double), ctr);
     }
     alloc_adjoint(*h, LBM_STORE_F32);
-    h->record.alloc(((size_t)N * 4 + CELL_PAD) * sizeof(float), ctr);
+    h->record.grow(((size_t)N * 4 + CELL_PAD) * sizeof(float), ctr, h->device, h->stream);
     // nonlinear ports transpose at the next state (the extrapolations at the
     // neighbours, the regularized port at the port cell): its (rho - 1, u)
     // record from one step into the other array, which leaves the current
@@ -2945,7 +2987,7 @@ lbm_status lbm_slab_step(lbm_handle* h, lbm_slab_diag_t* diag) {
     return guarded(h, [&]() {
         require_slab(*h);
         if (!h->state_valid) throw StateError("no current state: call lbm_slab_begin first");
-        h->diag.alloc(sizeof(StepDiag), &h->device_bytes);
+        h->diag.grow(sizeof(StepDiag), &h->device_bytes, h->device, h->stream);
         step(*h, h->diag.as<StepDiag>(), nullptr);
         read_slab_diag(*h, diag);
         h->forward_done = false;
@@ -2957,7 +2999,7 @@ lbm_status lbm_slab_inspect(lbm_handle* h, lbm_slab_diag_t* diag) {
     return guarded(h, [&]() {
         require_slab(*h);
         if (!h->state_valid) throw StateError("no current state: call lbm_slab_begin first");
-        h->diag.alloc(sizeof(StepDiag), &h->device_bytes);
+        h->diag.grow(sizeof(StepDiag), &h->device_bytes, h->device, h->stream);
         inspect(*h, h->diag.as<StepDiag>(), nullptr);
         read_slab_diag(*h, diag);
         h->forward_done = true;
@@ -3016,9 +3058,9 @@ lbm_status lbm_slab_adjoint_begin(lbm_handle* h, const double* weights, double* 
         alloc_adjoint(*h, LBM_STORE_F32);
         int64_t* ctr = &h->device_bytes;
         const int64_t n = h->n();
-        h->record.alloc(((size_t)n * 4 + CELL_PAD) * sizeof(float), ctr);
-        h->abar_final.alloc((size_t)n * 4, ctr);
-        h->phibar.alloc((size_t)n * 4, ctr);
+        h->record.grow(((size_t)n * 4 + CELL_PAD) * sizeof(float), ctr, h->device, h->stream);
+        h->abar_final.grow((size_t)n * 4, ctr, h->device, h->stream);
+        h->phibar.grow((size_t)n * 4, ctr, h->device, h->stream);
         delete h->slab_adj;
         h->slab_adj = new AdjState();  // unit scale: the values cross ranks as they are
         // cotangents of the ghost planes belong to other ranks
@@ -3077,7 +3119,7 @@ lbm_status lbm_design_vjp(lbm_handle* h, const double* phi_bar, double* out, siz
         require_design(*h);
         check_n(*h, n, (size_t)h->n(), "phi_bar");
         int64_t* ctr = &h->device_bytes;
-        h->phibar.alloc(n * 4, ctr);
+        h->phibar.grow(n * 4, ctr, h->device, h->stream);
         const PinLease pin(pin_bytes((int64_t)n));
         upload(*h, phi_bar, h->phibar.as<float>(), (int64_t)n, false);
         design_transpose(*h, h->phibar.as<float>(), nullptr, 1.f, nullptr);

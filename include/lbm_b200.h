@@ -254,7 +254,8 @@ typedef enum { LBM_CKPT_EVERY = 0, LBM_CKPT_BINOMIAL = 1 } lbm_checkpointing;
 typedef struct {
     int32_t mode;             /* lbm_adjoint_mode */
     int32_t lambda_storage;   /* lbm_storage of the adjoint populations */
-    int64_t checkpoint_every; /* HORIZON: K (<= 0 selects sqrt(step_count)) */
+    int64_t checkpoint_every; /* HORIZON: K (<= 0: every record of the trajectory is kept where they fit in
+                                 16 GB and half of the free memory, else K = sqrt(step_count)) */
     int64_t max_iterations;   /* STEADY: cap */
     int64_t check_every;      /* STEADY: residual readback period */
     double tolerance;         /* STEADY: relative residual */

@@ -11,7 +11,7 @@ the other way: one unit of the storage format (2^-11, 2^-8) of (f - w)/w.
 import numpy as np
 import pytest
 
-from implexity_b200 import LbmSolver, workloads
+from implexity_b200 import ContractError, LbmSolver, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -45,10 +45,12 @@ def regularized(shape):
 
 
 CASES = {
-    # one block; several blocks of 128; one cell per thread over 256-thread blocks; several cells per thread
+    # one block; several blocks of 128; one cell per thread over 256-thread blocks, two and three per SM;
+    # several cells per thread
     "8x6x5": channel((8, 6, 5), "D3Q19", "bgk", "float32"),
     "23x17x13_mrt": channel((23, 17, 13), "D3Q19", "mrt", "float32"),
     "41x31x29_q27": channel((41, 31, 29), "D3Q27", "trt", "float32"),
+    "53x45x43": channel((53, 45, 43), "D3Q19", "trt", "float32"),
     "67x45x43": channel((67, 45, 43), "D3Q19", "trt", "float32"),
     "67x45x43_f16": channel((67, 45, 43), "D3Q19", "trt", "float16"),
     "19x11x9_bf16": channel((19, 11, 9), "D3Q27", "mrt", "bfloat16"),
@@ -147,3 +149,57 @@ def test_kept_records_match_recomputed_ones(gpu_lib, objective):
     assert kept.iterations == ck.iterations == T
     assert rel_l2(g, g_ck) <= 1e-6
     assert rel_l2(g, g_one) <= 2e-5
+
+
+def test_staged_sums_across_chunks(gpu_lib):
+    """Staged steps combine the partials of sixteen steps at a time: response
+    sums and admission records of every state of a longer run, against the
+    responses of each state (FP32 per cell against FP64) and single steps."""
+    steps = 21
+    prob = workloads.pulsatile_problem(shape=(11, 8, 7), steps=steps, lattice="D3Q19", period_steps=9)
+    prob["ports"][1]["reconstruction"] = "non_equilibrium_extrapolation"  # a run of steps does not take it
+    prob["design_region"][-2] = False
+    with LbmSolver(prob) as s:
+        s.set_design(workloads.uniform_design((11, 8, 7), 3))
+        s.forward()
+        mean, tr = s.time_average(), s.trajectory()
+        acc = np.zeros(8)
+        for t in range(1, steps + 1):
+            s.forward(t)
+            acc += s.responses() / steps
+            one = s.trajectory()
+            for k in ("mass", "min_population", "max_speed", "exchange"):
+                assert one[k][t] == tr[k][t], (k, t)
+    assert np.allclose(mean[[0, 3, 4, 5, 6, 7]], acc[[0, 3, 4, 5, 6, 7]], rtol=1e-5)
+
+
+@pytest.mark.parametrize("shape", [(9, 8, 7), (40, 26, 24)])
+def test_refused_design_keeps_the_last_map(gpu_lib, shape):
+    """Checked on the host (504 cells) and on the device (24 960 cells)."""
+    prob = workloads.channel_problem(shape=shape, steps=3)
+    good = workloads.uniform_design(shape, 2)
+    with LbmSolver(prob) as s:
+        s.set_design(good)
+        phi, alpha = s.design()
+        for bad_value in (np.nan, 1.0 + 1e-9, -1e-300, np.inf):
+            bad = workloads.uniform_design(shape, 5)
+            bad[-1, -1, -1] = bad_value
+            with pytest.raises(ContractError):
+                s.set_design(bad)
+        phi2, alpha2 = s.design()
+        s.set_design(good)
+        phi3, _ = s.design()
+    assert np.array_equal(phi, phi2) and np.array_equal(alpha, alpha2) and np.array_equal(phi, phi3)
+
+
+@pytest.mark.parametrize("lattice,shape", [("D3Q19", (5, 4, 3)), ("D3Q27", (17, 16, 15)), ("D3Q19", (96, 80, 64))])
+def test_population_round_trip(gpu_lib, lattice, shape):
+    """Less than a block, a partial last block, and more cells than one piece
+    of the staging holds (441 505); g = f - w is kept in FP32, 2^-24 of 0.02."""
+    q, n = int(lattice[3:]), int(np.prod(shape))
+    prob = workloads.channel_problem(shape=shape, steps=1, lattice=lattice, ports=False)
+    f = 0.05 + 0.02 * np.random.default_rng(0).uniform(-1.0, 1.0, (n, q))
+    with LbmSolver(prob) as s:
+        s.set_populations(f)
+        back = s.populations()
+    assert np.max(np.abs(back - f)) <= 2.0**-24
