@@ -119,11 +119,13 @@ __device__ __forceinline__ void adj_one_cell(const AdjArgs& a, const S* st, int 
 
 // STG = 1: the stage-objective variant, which reads the second moments of
 // the recorded state as well and adds the state's response VJP.
-// Residency: D3Q19 with 16-bit storage runs three blocks per SM (72
-// registers): its step is bound by latency and instruction issue, not bytes,
-// and a third block's warps hide more of it; the others keep two blocks.
+// Residency: 16-bit storage runs three blocks per SM (72 registers): its step
+// is bound by latency and instruction issue, not bytes, and a third block's
+// warps hide more of it (us per step with two / three, FP16: 256x128x128 114.0 /
+// 101.5, 128^3 63.6 / 52.9, D3Q27 192x128x128 120.1 / 109.3, with the registers
+// spilled).  FP32 storage keeps two (135.1 / 135.9, 71.6 / 72.4).
 template <int Q, int COLL, typename T, int AL, int STG>
-__global__ void __launch_bounds__(TPB, (sizeof(T) == 2 && Q == 19 ? 3 : 2)) k_adjoint(AdjArgs a) {
+__global__ void __launch_bounds__(TPB, (sizeof(T) == 2 ? 3 : 2)) k_adjoint(AdjArgs a) {
     constexpr int NREC = STG ? 10 : 4;
     using S = AdjStage<Q, T, NREC>;
     constexpr int NCOPY = Q + NREC + 2;  // runs of lambda, the record, mask and alpha

@@ -1259,6 +1259,8 @@ void inspect(lbm_handle& h, StepDiag* diag, float* record, bool record_s = false
 //   adjoint FP32            8.3 / 3.1   14.2 / 9.0  24.9 / 23.9  30.6 / 33.7
 //   adjoint FP16            8.3 / 3.2   12.4 / 9.2  20.6 / 17.4  24.7 / 21.9  32.5 / 35.5
 //   adjoint D3Q27          10.3 / 4.0  18.5 / 12.2  40.1 / 34.6  43.8 / 42.6  54.1 / 53.3  99.2 / 103
+//   adjoint D3Q27 FP16     12.4 / 4.1  20.6 / 12.4  34.5 / 25.5  40.7 / 35.6  47.3 / 44.7  84.2 / 86.0
+// (the last before a third block per SM took 8% off its staged step)
 // and with the response sums 20.0 / 15.4 (262 144, FP32), 33.7 / 36.3 (614 400),
 // D3Q27 53.4 / 45.9 and 68.0 / 67.7 (1 032 192); with the stage seeds (a dozen
 // divisions per cell then) 24.0 / 22.9 and 47.4 / 52.6, D3Q27 30.2 / 26.2 and
@@ -1267,7 +1269,7 @@ void inspect(lbm_handle& h, StepDiag* diag, float* record, bool record_s = false
 bool marches(const lbm_handle& h, bool adjoint, bool stage) {
     const bool wide = (adjoint ? h.lam_storage : h.storage) == LBM_STORE_F32, q27 = h.Q == 27;
     int64_t most;
-    if (adjoint) most = stage ? 400 << 10 : q27 ? 1 << 20 : wide ? 640 << 10 : 900 << 10;
+    if (adjoint) most = stage ? 400 << 10 : !wide ? 900 << 10 : q27 ? 1 << 20 : 640 << 10;
     else if (!wide) most = stage && !q27 ? 1 << 20 : 4 << 20;
     else if (h.collision_fp64) most = 2 << 20;
     else most = q27 ? 900 << 10 : stage ? 400 << 10 : 640 << 10;
