@@ -328,13 +328,12 @@ void reconstruct(const HostLat& L, const PortSpec& p, const double a[3], const d
 }
 
 // ------------------------------------------------------------ device buffers
-// Checkpoints come from one stream-ordered pool per device instead of
-// cudaMalloc / cudaFree on every gradient: on a shared host those took 20 to
-// 100 ms for a horizon gradient's sixteen 320 MB states and varied with the
-// neighbours' load.  Freed states stay in the pool up to POOL_KEEP bytes, for
-// the next gradient of any handle (the frees are ordered on the owner's
-// stream, the driver orders a reuse on another); a failing allocation gives
-// them back first.
+// Handles' buffers and checkpoints come from one stream-ordered pool per
+// device.  With cudaMalloc / cudaFree on every gradient, the sixteen 320 MB
+// states of a horizon gradient cost 20 to 100 ms on a shared host, by the
+// neighbours' load.  Freed memory stays in the pool up to POOL_KEEP bytes, for
+// the next gradient or handle (the frees are ordered on the owner's stream, the
+// driver orders a reuse on another); a failing allocation gives it back first.
 constexpr uint64_t POOL_KEEP = 16ull << 30;
 
 cudaMemPool_t state_pool(int device) {
@@ -1111,21 +1110,21 @@ void validate_and_build(lbm_handle& h, const lbm_problem_t& p) {
     CK(cudaEventCreate(&h.ev0));
     CK(cudaEventCreate(&h.ev1));
     int64_t* ctr = &h.device_bytes;
-    h.pop.alloc(2 * h.array_bytes(h.storage), ctr);
-    h.mask.alloc((size_t)(n + CELL_PAD) * 4, ctr);
-    h.alpha.alloc((size_t)(n + CELL_PAD) * 4, ctr);
-    h.errflag.alloc(3 * 64 * sizeof(int), ctr);
-    h.phi.alloc((size_t)n * 4, ctr);
-    h.raw.alloc((size_t)n * 4, ctr);
-    h.den.alloc((size_t)n * 4, ctr);
-    h.slope.alloc((size_t)n * 4, ctr);
-    h.cls_d.alloc((size_t)n, ctr);
-    h.fixed_d.alloc((size_t)n * 4, ctr);
-    h.offsets_d.alloc(std::max<size_t>(1, h.offsets.size()) * sizeof(int4), ctr);
-    h.ports_d.alloc(std::max<size_t>(1, maps.size()) * sizeof(PortMap), ctr);
-    h.partial.alloc((size_t)h.sms * 32 * 16 * sizeof(double), ctr);
-    h.counter.alloc(2 * sizeof(unsigned), ctr);  // [0] step/objective sums, [1] fused response sums
-    h.sums.alloc(64 * sizeof(double), ctr);
+    h.pop.grow(2 * h.array_bytes(h.storage), ctr, h.device, h.stream);
+    h.mask.grow((size_t)(n + CELL_PAD) * 4, ctr, h.device, h.stream);
+    h.alpha.grow((size_t)(n + CELL_PAD) * 4, ctr, h.device, h.stream);
+    h.errflag.grow(3 * 64 * sizeof(int), ctr, h.device, h.stream);
+    h.phi.grow((size_t)n * 4, ctr, h.device, h.stream);
+    h.raw.grow((size_t)n * 4, ctr, h.device, h.stream);
+    h.den.grow((size_t)n * 4, ctr, h.device, h.stream);
+    h.slope.grow((size_t)n * 4, ctr, h.device, h.stream);
+    h.cls_d.grow((size_t)n, ctr, h.device, h.stream);
+    h.fixed_d.grow((size_t)n * 4, ctr, h.device, h.stream);
+    h.offsets_d.grow(std::max<size_t>(1, h.offsets.size()) * sizeof(int4), ctr, h.device, h.stream);
+    h.ports_d.grow(std::max<size_t>(1, maps.size()) * sizeof(PortMap), ctr, h.device, h.stream);
+    h.partial.grow((size_t)h.sms * 32 * 16 * sizeof(double), ctr, h.device, h.stream);
+    h.counter.grow(2 * sizeof(unsigned), ctr, h.device, h.stream);  // [0] step/objective sums, [1] fused response sums
+    h.sums.grow(64 * sizeof(double), ctr, h.device, h.stream);
     CK(cudaMemsetAsync(h.mask.p, 0xff, (size_t)(n + CELL_PAD) * 4, h.stream));  // padding reads as solid
     CK(cudaMemcpyAsync(h.mask.p, mask.data(), (size_t)n * 4, cudaMemcpyHostToDevice, h.stream));
     CK(cudaMemsetAsync(h.alpha.p, 0, (size_t)(n + CELL_PAD) * 4, h.stream));
@@ -1135,7 +1134,7 @@ void validate_and_build(lbm_handle& h, const lbm_problem_t& p) {
         CK(cudaMemcpyAsync(h.offsets_d.p, h.offsets.data(), h.offsets.size() * sizeof(int4), cudaMemcpyHostToDevice,
                            h.stream));
     if (!nee_cells.empty()) {
-        h.nee_cells_d.alloc(nee_cells.size() * sizeof(uint32_t), ctr);
+        h.nee_cells_d.grow(nee_cells.size() * sizeof(uint32_t), ctr, h.device, h.stream);
         CK(cudaMemcpyAsync(h.nee_cells_d.p, nee_cells.data(), nee_cells.size() * sizeof(uint32_t),
                            cudaMemcpyHostToDevice, h.stream));
     }
@@ -2393,8 +2392,10 @@ void lbm_destroy(lbm_handle* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     h->ckpts.clear();
     // the pool's buffers go back in the order of the stream, before it goes
-    for (DevBuf* b : {&h->lam, &h->record, &h->abar, &h->abar_final, &h->phibar, &h->scale, &h->grad, &h->scratch, &h->diag,
-                      &h->tsums})
+    for (DevBuf* b : {&h->pop, &h->mask, &h->alpha, &h->phi, &h->raw, &h->den, &h->slope, &h->cls_d, &h->fixed_d,
+                      &h->offsets_d, &h->ports_d, &h->partial, &h->counter, &h->sums, &h->errflag, &h->nee_cells_d,
+                      &h->lam, &h->record, &h->abar, &h->abar_final, &h->phibar, &h->scale, &h->grad, &h->scratch,
+                      &h->diag, &h->tsums})
         b->reset();
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
