@@ -74,7 +74,8 @@ __device__ __forceinline__ void adj_one_cell(const AdjArgs& a, const S* st, int 
     float om = a.P.omega, omm = a.P.om;
     if (a.omega_cell) om = omm = a.omega_cell[x];  // Tau::PerCell (BGK only)
     const bool post = (STG && a.stage) || (a.port_transpose && (m & MASK_PORT));
-    float ab = collide_vjp<Q, COLL>(v, rp, u, st->alpha[c], a.P, om, omm, post ? 1.f : k_out) * a.in_scale_inv;
+    float ab = collide_vjp<Q, COLL, sizeof(T) == 2>(v, rp, u, st->alpha[c], a.P, om, omm, post ? 1.f : k_out) *
+               a.in_scale_inv;
     if constexpr (STG) {
         if (a.stage) {
             // the stage seed of this state: d(w . responses)/dg from its record
@@ -82,8 +83,8 @@ __device__ __forceinline__ void adj_one_cell(const AdjArgs& a, const S* st, int 
 #pragma unroll
             for (int e = 0; e < 6; ++e) Sm[e] = st->rec[4 + e][a.recd[4 + e] + c];
             const PortMap* pm = (m & MASK_PORT) ? &a.ports[((m >> MASK_PORT_SHIFT) & 7u) - 1] : nullptr;
-            ab += response_vjp<Q>(rp, u, Sm, st->alpha[c], pm ? pm->dp_weight : 0.f, pm != nullptr, a.seed,
-                                  a.P, fb);
+            ab += response_vjp<Q, sizeof(T) == 2>(rp, u, Sm, st->alpha[c], pm ? pm->dp_weight : 0.f, pm != nullptr,
+                                                  a.seed, a.P, fb);
 #pragma unroll
             for (int q = 0; q < Q; ++q) v[q] = fmaf(fb[q], s_in, v[q]);
         }

@@ -985,7 +985,14 @@ __device__ __forceinline__ Macro collide_fused_dp(float (&vf)[Q], float alpha_f,
 // (even / odd), taken pair by pair; the MRT rank-one terms add analytic
 // multiples of the precomputed moments of their basis vectors.  Then the
 // Brinkman chain F = rho (a - alpha u), u = (m/rho + a/2)/(1 + alpha/2).
-template <int Q, int COLL>
+//
+// HALF: the cotangent is stored in 16 bits.  Its values round every step, so
+// another order of these operations gives another trajectory, off by the
+// storage's noise: like the 16-bit forward step (collide_fused) this one keeps
+// its order, the moments of gb itself and the cotangents of eq, src and the
+// Brinkman chain in turn.  (The collected form would take 101 us of an FP16 step
+// of 256x128x128 cells where this one takes 110.)
+template <int Q, int COLL, bool HALF>
 __device__ __forceinline__ float collide_vjp(float (&gb)[Q], float rp, const float (&u)[3], float alpha,
                                              const Physics& P, float om, float omm, float k = 1.f) {
     using L = Lat<Q>;
@@ -1001,15 +1008,15 @@ __device__ __forceinline__ float collide_vjp(float (&gb)[Q], float rp, const flo
     // That takes the cancellations out of the moments: the FP32 bias of a step
     // in the mass mode falls from 1.9e-8 to under 1e-9 of r, the alpha
     // cotangent's error by a factor of ten.
-    const float r = gb[0];
-    float M0 = 0.f;
+    const float r = HALF ? 0.f : gb[0];
+    float M0 = HALF ? L::w(0) * gb[0] : 0.f;
     float M1[3] = {0.f, 0.f, 0.f}, M2[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     float SM[NP], DF[NP];
-    float g0 = 0.f;  // the rest population's output, less rho_bar and r
+    float g0 = HALF ? (1.f - om) * gb[0] : 0.f;  // the rest population's output, less rho_bar and r
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
         const int i = k + 1, o = opp<Q>(i);
-        const float sm = fmaf(-2.f, r, gb[i] + gb[o]), df = gb[i] - gb[o];
+        const float sm = HALF ? gb[i] + gb[o] : fmaf(-2.f, r, gb[i] + gb[o]), df = gb[i] - gb[o];
         SM[k] = sm;
         DF[k] = df;
         const float w = L::w(i);
@@ -1031,115 +1038,203 @@ __device__ __forceinline__ float collide_vjp(float (&gb)[Q], float rp, const flo
         if (c0 && c2) M2[4] = fmaf(w * c0 * c2, sm, M2[4]);
         if (c1 && c2) M2[5] = fmaf(w * c1 * c2, sm, M2[5]);
     }
-    // The cotangents of (rho, u, F) and the Brinkman chain, collected.  With
-    //   e  = 9 M2 u - 3 M0 u,  ea = 9 M2 a - 3 M0 a
-    // (the equilibrium's and the source's second-order terms) and hz, ho = 1 -
-    // om/2, 1 - omm/2, the force F = rho (a - alpha u) makes every term a
-    // multiple of M1, e and ea:
-    //   F_bar = 3 ho M1 + hz e
-    //   u_bar = rho [(om - 2 hz alpha) e + 3 (omm - ho alpha) M1 + hz ea]
-    //   rho_bar = om M0 + om/2 u.e + 3 omm u.M1 + F_bar.(a - alpha u) - m_bar.(s u - a/2)
-    //   m_bar = u_bar / (rho s)
-    // An even MRT correction adds its moments D0, D2 to those of the relaxed
-    // part and takes half of them from the source's: with e' = 9 D2 u - 3 D0 u
-    // and ea' likewise, F_bar -= e'/2, u_bar += rho [(1 + alpha) e' - ea'/2],
-    // rho_bar += D0 + u.e'/2.
-    const float hz = 1.f - 0.5f * om, ho = 1.f - 0.5f * omm;
-    const bool forced = P.a[0] != 0.f || P.a[1] != 0.f || P.a[2] != 0.f;  // the same for every cell
+    float bulk_c = 0.f;     // MRT_BULK: the bulk correction's coefficient
+    float cproj[MAX_PROJ];  // MRT: the rank-one corrections' coefficients
+    float rho_bar, abar, mb[3];
     // symmetric 3x3 stored xx yy zz xy xz yz
     auto mul = [](const float (&S)[6], const float* v, float* out) {
         out[0] = S[0] * v[0] + S[3] * v[1] + S[4] * v[2];
         out[1] = S[3] * v[0] + S[1] * v[1] + S[5] * v[2];
         out[2] = S[4] * v[0] + S[5] * v[1] + S[2] * v[2];
     };
-    float e[3];
-    mul(M2, u, e);
-    const float M03 = 3.f * M0;
+    if constexpr (HALF) {
+        float F[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) e[d] = fmaf(9.f, e[d], -M03 * u[d]);
-    float bulk_c = 0.f;     // MRT_BULK: the bulk correction's coefficient
-    float cproj[MAX_PROJ];  // MRT: the rank-one corrections' coefficients
-    float D0 = 0.f, ep[3] = {0.f, 0.f, 0.f}, eap[3] = {0.f, 0.f, 0.f};
-    if constexpr (COLL == CK_MRT_BULK) {
-        // the bulk correction folded: b_i = |c_i|^2 - 1, |b|^2_W = 2/3,
-        // sum_i w_i b_i = 0 and sum_i w_i b_i c_ia c_ib = 2/9 delta_ab on both lattices
-        float b = 0.f;
-#pragma unroll
-        for (int k = 0; k < NP; ++k) {
-            const int i = k + 1;
-            const int c2 = L::cx(i) * L::cx(i) + L::cy(i) * L::cy(i) + L::cz(i) * L::cz(i);
-            if (c2 != 1) b = fmaf(L::w(i) * (float)(c2 - 1), SM[k], b);  // folded after unrolling
-        }
-        bulk_c = P.proj_rate[0] * b * 1.5f;
-        g0 += bulk_c;
+        for (int d = 0; d < 3; ++d) F[d] = rho * (P.a[d] - alpha * u[d]);
+        float Z0 = om * M0, H0 = (1.f - 0.5f * om) * M0;
+        float Z1[3], H1[3], Z2[6], H2[6];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            ep[d] = 2.f * bulk_c * u[d];
-            eap[d] = 2.f * bulk_c * P.a[d];
+            Z1[d] = omm * M1[d];
+            H1[d] = (1.f - 0.5f * omm) * M1[d];
         }
-    }
-    if constexpr (COLL == CK_MRT) {
-        float D2[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int p = 0; p < MAX_PROJ; ++p) {
-            cproj[p] = 0.f;
-            if (p < P.n_proj) {
-                float b = 0.f;
+        for (int e = 0; e < 6; ++e) {
+            Z2[e] = om * M2[e];
+            H2[e] = (1.f - 0.5f * om) * M2[e];
+        }
+        if constexpr (COLL == CK_MRT_BULK) {
+            // the bulk correction folded: b_i = |c_i|^2 - 1, |b|^2_W = 2/3,
+            // sum_i w_i b_i = 0 and sum_i w_i b_i c_ia c_ib = 2/9 delta_ab on both lattices
+            float e = -L::w(0) * gb[0];
 #pragma unroll
-                for (int i = 1; i < Q; ++i) b = fmaf(P.proj_left[p][i], gb[i] - r, b);
-                const float c = P.proj_rate[p] * b;
-                cproj[p] = c;
-                g0 = fmaf(-c, P.proj_right[p][0], g0);
-                D0 = fmaf(c, P.proj_m0[p], D0);
+            for (int k = 0; k < NP; ++k) {
+                const int i = k + 1;
+                const int c2 = L::cx(i) * L::cx(i) + L::cy(i) * L::cy(i) + L::cz(i) * L::cz(i);
+                if (c2 != 1) e = fmaf(L::w(i) * (float)(c2 - 1), SM[k], e);  // folded after unrolling
+            }
+            bulk_c = P.proj_rate[0] * e * 1.5f;
+            const float c = bulk_c;
+            g0 += c;
 #pragma unroll
-                for (int e2 = 0; e2 < 6; ++e2) D2[e2] = fmaf(c, P.proj_m2[p][e2], D2[e2]);
+            for (int d = 0; d < 3; ++d) {
+                Z2[d] = fmaf(c, 2.f / 9.f, Z2[d]);
+                H2[d] = fmaf(-0.5f * c, 2.f / 9.f, H2[d]);
             }
         }
-        mul(D2, u, ep);
-        mul(D2, P.a, eap);
+        if constexpr (COLL == CK_MRT) {
+#pragma unroll
+            for (int p = 0; p < MAX_PROJ; ++p) {
+                cproj[p] = 0.f;
+                if (p < P.n_proj) {
+                    float e = 0.f;
+#pragma unroll
+                    for (int i = 0; i < Q; ++i) e = fmaf(P.proj_left[p][i], gb[i], e);
+                    const float c = P.proj_rate[p] * e;
+                    cproj[p] = c;
+                    g0 = fmaf(-c, P.proj_right[p][0], g0);
+                    Z0 = fmaf(c, P.proj_m0[p], Z0);
+                    H0 = fmaf(-0.5f * c, P.proj_m0[p], H0);
+#pragma unroll
+                    for (int e2 = 0; e2 < 6; ++e2) {
+                        Z2[e2] = fmaf(c, P.proj_m2[p][e2], Z2[e2]);
+                        H2[e2] = fmaf(-0.5f * c, P.proj_m2[p][e2], H2[e2]);
+                    }
+                }
+            }
+        }
+        float Z2u[3], H2u[3], H2F[3];
+        mul(Z2, u, Z2u);
+        mul(H2, u, H2u);
+        mul(H2, F, H2F);
+        const float usq = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
+        rho_bar = Z0 * (1.f - 1.5f * usq) + 3.f * (u[0] * Z1[0] + u[1] * Z1[1] + u[2] * Z1[2]) +
+                        4.5f * (u[0] * Z2u[0] + u[1] * Z2u[1] + u[2] * Z2u[2]);
+        float ub[3], Fb[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            ep[d] = fmaf(9.f, ep[d], -3.f * D0 * u[d]);
-            eap[d] = fmaf(9.f, eap[d], -3.f * D0 * P.a[d]);
+            ub[d] = rho * (3.f * Z1[d] + 9.f * Z2u[d] - 3.f * u[d] * Z0) + 9.f * H2F[d] - 3.f * F[d] * H0;
+            Fb[d] = 3.f * H1[d] + 9.f * H2u[d] - 3.f * u[d] * H0;
         }
-    }
-    const float ce = fmaf(-2.f * hz, alpha, om), cm1 = 3.f * fmaf(-ho, alpha, omm), ho3 = 3.f * ho;
-    float Fb[3], ur[3];  // F_bar and u_bar / rho
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        Fb[d] = fmaf(hz, e[d], ho3 * M1[d]);
-        ur[d] = fmaf(ce, e[d], cm1 * M1[d]);
-        if constexpr (COLL == CK_MRT_BULK || COLL == CK_MRT) {
-            Fb[d] = fmaf(-0.5f, ep[d], Fb[d]);
-            ur[d] = fmaf(1.f + alpha, ep[d], ur[d]);
-        }
-    }
-    if (forced) {
-        float ea[3];
-        mul(M2, P.a, ea);
+        abar = 0.f;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            ur[d] = fmaf(hz, fmaf(9.f, ea[d], -M03 * P.a[d]), ur[d]);
-            if constexpr (COLL == CK_MRT_BULK || COLL == CK_MRT) ur[d] = fmaf(-0.5f, eap[d], ur[d]);
+            rho_bar += Fb[d] * (P.a[d] - alpha * u[d]);
+            abar -= rho * Fb[d] * u[d];
+            ub[d] -= rho * alpha * Fb[d];
         }
-    }
-    auto dot = [](const float* x, const float* y) { return fmaf(x[2], y[2], fmaf(x[1], y[1], x[0] * y[0])); };
-    const float fu = dot(Fb, u), wu = dot(ur, u);
-    float rho_bar = fmaf(om, fmaf(0.5f, dot(u, e), M0), 3.f * omm * dot(u, M1)) - fmaf(alpha, fu, wu);
-    if constexpr (COLL == CK_MRT_BULK || COLL == CK_MRT) rho_bar += fmaf(0.5f, dot(u, ep), D0);
-    const float inv_s = __fdividef(1.f, s);
-    float mb[3];
+        const float inv_s = __fdividef(1.f, s);
+        const float inv = __fdividef(inv_s, rho);
+        float sbar = 0.f;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) mb[d] = ur[d] * inv_s;
-    if (forced) rho_bar += dot(Fb, P.a) + 0.5f * dot(mb, P.a);
-    // d/d alpha: -rho F_bar.u through F, -u_bar.u / (2 s) through u
-    const float abar = -rho * fmaf(0.5f * inv_s, wu, fu);
+        for (int d = 0; d < 3; ++d) {
+            mb[d] = ub[d] * inv;
+            rho_bar -= ub[d] * (s * u[d] - 0.5f * P.a[d]) * inv;
+            sbar -= ub[d] * u[d] * inv_s;
+        }
+        abar += 0.5f * sbar;
+    } else {
+        // The cotangents of (rho, u, F) and the Brinkman chain, collected.  With
+        //   e  = 9 M2 u - 3 M0 u,  ea = 9 M2 a - 3 M0 a
+        // (the equilibrium's and the source's second-order terms) and hz, ho = 1 -
+        // om/2, 1 - omm/2, the force F = rho (a - alpha u) makes every term a
+        // multiple of M1, e and ea:
+        //   F_bar = 3 ho M1 + hz e
+        //   u_bar = rho [(om - 2 hz alpha) e + 3 (omm - ho alpha) M1 + hz ea]
+        //   rho_bar = om M0 + om/2 u.e + 3 omm u.M1 + F_bar.(a - alpha u) - m_bar.(s u - a/2)
+        //   m_bar = u_bar / (rho s)
+        // An even MRT correction adds its moments D0, D2 to those of the relaxed
+        // part and takes half of them from the source's: with e' = 9 D2 u - 3 D0 u
+        // and ea' likewise, F_bar -= e'/2, u_bar += rho [(1 + alpha) e' - ea'/2],
+        // rho_bar += D0 + u.e'/2.
+        const float hz = 1.f - 0.5f * om, ho = 1.f - 0.5f * omm;
+        const bool forced = P.a[0] != 0.f || P.a[1] != 0.f || P.a[2] != 0.f;  // the same for every cell
+        float e[3];
+        mul(M2, u, e);
+        const float M03 = 3.f * M0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) e[d] = fmaf(9.f, e[d], -M03 * u[d]);
+        float D0 = 0.f, ep[3] = {0.f, 0.f, 0.f}, eap[3] = {0.f, 0.f, 0.f};
+        if constexpr (COLL == CK_MRT_BULK) {
+            // the bulk correction folded: b_i = |c_i|^2 - 1, |b|^2_W = 2/3,
+            // sum_i w_i b_i = 0 and sum_i w_i b_i c_ia c_ib = 2/9 delta_ab on both lattices
+            float b = 0.f;
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                const int i = k + 1;
+                const int c2 = L::cx(i) * L::cx(i) + L::cy(i) * L::cy(i) + L::cz(i) * L::cz(i);
+                if (c2 != 1) b = fmaf(L::w(i) * (float)(c2 - 1), SM[k], b);  // folded after unrolling
+            }
+            bulk_c = P.proj_rate[0] * b * 1.5f;
+            g0 += bulk_c;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                ep[d] = 2.f * bulk_c * u[d];
+                eap[d] = 2.f * bulk_c * P.a[d];
+            }
+        }
+        if constexpr (COLL == CK_MRT) {
+            float D2[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int p = 0; p < MAX_PROJ; ++p) {
+                cproj[p] = 0.f;
+                if (p < P.n_proj) {
+                    float b = 0.f;
+#pragma unroll
+                    for (int i = 1; i < Q; ++i) b = fmaf(P.proj_left[p][i], gb[i] - r, b);
+                    const float c = P.proj_rate[p] * b;
+                    cproj[p] = c;
+                    g0 = fmaf(-c, P.proj_right[p][0], g0);
+                    D0 = fmaf(c, P.proj_m0[p], D0);
+#pragma unroll
+                    for (int e2 = 0; e2 < 6; ++e2) D2[e2] = fmaf(c, P.proj_m2[p][e2], D2[e2]);
+                }
+            }
+            mul(D2, u, ep);
+            mul(D2, P.a, eap);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                ep[d] = fmaf(9.f, ep[d], -3.f * D0 * u[d]);
+                eap[d] = fmaf(9.f, eap[d], -3.f * D0 * P.a[d]);
+            }
+        }
+        const float ce = fmaf(-2.f * hz, alpha, om), cm1 = 3.f * fmaf(-ho, alpha, omm), ho3 = 3.f * ho;
+        float Fb[3], ur[3];  // F_bar and u_bar / rho
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            Fb[d] = fmaf(hz, e[d], ho3 * M1[d]);
+            ur[d] = fmaf(ce, e[d], cm1 * M1[d]);
+            if constexpr (COLL == CK_MRT_BULK || COLL == CK_MRT) {
+                Fb[d] = fmaf(-0.5f, ep[d], Fb[d]);
+                ur[d] = fmaf(1.f + alpha, ep[d], ur[d]);
+            }
+        }
+        if (forced) {
+            float ea[3];
+            mul(M2, P.a, ea);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                ur[d] = fmaf(hz, fmaf(9.f, ea[d], -M03 * P.a[d]), ur[d]);
+                if constexpr (COLL == CK_MRT_BULK || COLL == CK_MRT) ur[d] = fmaf(-0.5f, eap[d], ur[d]);
+            }
+        }
+        auto dot = [](const float* x, const float* y) { return fmaf(x[2], y[2], fmaf(x[1], y[1], x[0] * y[0])); };
+        const float fu = dot(Fb, u), wu = dot(ur, u);
+        rho_bar = fmaf(om, fmaf(0.5f, dot(u, e), M0), 3.f * omm * dot(u, M1)) - fmaf(alpha, fu, wu);
+        if constexpr (COLL == CK_MRT_BULK || COLL == CK_MRT) rho_bar += fmaf(0.5f, dot(u, ep), D0);
+        const float inv_s = __fdividef(1.f, s);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) mb[d] = ur[d] * inv_s;
+        if (forced) rho_bar += dot(Fb, P.a) + 0.5f * dot(mb, P.a);
+        // d/d alpha: -rho F_bar.u through F, -u_bar.u / (2 s) through u
+        abar = -rho * fmaf(0.5f * inv_s, wu, fu);
+    }
     // output, times k: gb - R^T gb + rho_bar + c . mb, pair by pair (with
     // the MRT corrections, which are even: the same for i and opp(i)); the
     // scale k of the stored cotangent enters the few per-cell coefficients
     // instead of every population
     const float hp = 0.5f * (1.f - om) * k, hm = 0.5f * (1.f - omm) * k;
-    const float kr = k * (rho_bar + r), kbulk = k * bulk_c;
+    const float kr = HALF ? k * rho_bar : k * (rho_bar + r), kbulk = k * bulk_c;
     float kmb[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) kmb[d] = k * mb[d];
@@ -1208,7 +1303,10 @@ __device__ __forceinline__ void second_moments(const float (&g)[Q], float (&S)[6
 // the Brinkman velocity u and the second moments S of g.  fb = d/dg; returns
 // the cotangent of alpha.  The responses depend on g only through these
 // moments, so the adjoint step can seed a state from its record alone.
-template <int Q>
+// HALF: the seed enters a cotangent stored in 16 bits, whose trajectories keep
+// their order of operations (collide_vjp), a dozen divisions per cell and all
+// (267 us per seeded FP16 step of 256x128x128 cells, 161 without them).
+template <int Q, bool HALF>
 __device__ __forceinline__ float response_vjp(float rp, const float (&u)[3], const float (&S)[6], float alpha,
                                               float dpw, bool port, const SeedParams& sp, const Physics& P,
                                               float (&fb)[Q]) {
@@ -1216,6 +1314,7 @@ __device__ __forceinline__ float response_vjp(float rp, const float (&u)[3], con
     const float k = sp.visc_k;
     const float rho = 1.f + rp;
     const float ir = 1.f / rho;
+    [[maybe_unused]] const float nu = (sp.tau - 0.5f) / 3.f;
     float F[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) F[d] = rho * (P.a[d] - alpha * u[d]);
@@ -1224,7 +1323,7 @@ __device__ __forceinline__ float response_vjp(float rp, const float (&u)[3], con
     float ss = 0.f;
 #pragma unroll
     for (int e = 0; e < 6; ++e) {
-        const float pi = S[e] - (e < 3 ? rp * (1.f / 3.f) : 0.f) - rho * u[ia[e]] * u[ib[e]];
+        const float pi = S[e] - (e < 3 ? (HALF ? rp / 3.f : rp * (1.f / 3.f)) : 0.f) - rho * u[ia[e]] * u[ib[e]];
         const float t = 0.5f * (u[ia[e]] * F[ib[e]] + u[ib[e]] * F[ia[e]]);
         sig[e] = -k * (pi + t);
         ss += (e < 3 ? 1.f : 2.f) * sig[e] * sig[e];
@@ -1236,19 +1335,23 @@ __device__ __forceinline__ float response_vjp(float rp, const float (&u)[3], con
     const float R = rho * sp.dens;
     const float W3 = sp.w[3], W4 = sp.w[4], W7 = sp.w[7];
     float rb = 0.f, abar = 0.f, ub[3], Fb[3] = {0.f, 0.f, 0.f}, Sb[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const float kin = W3 + W4 * alpha * sp.inv_dt;
+    const float kin = W3 + (HALF ? W4 * alpha / sp.dt_s : W4 * alpha * sp.inv_dt);
 #pragma unroll
     for (int d = 0; d < 3; ++d) ub[d] = sp.w[d] * V + kin * R * 2.f * U[d] * V;
     rb += kin * sp.dens * usq;
-    abar += W4 * R * sp.inv_dt * usq;
-    if (port) rb += sp.w[6] * dpw * sp.dens * V * V * (1.f / 3.f);
+    abar += (HALF ? W4 * R / sp.dt_s : W4 * R * sp.inv_dt) * usq;
+    if (port) {
+        const float pv = sp.w[6] * dpw * sp.dens * V * V;
+        rb += HALF ? pv / 3.f : pv * (1.f / 3.f);
+    }
     if (W7 != 0.f) {
         const float wv = W7 * sp.inv_nu * ir, kw = -k * wv;
-        rb -= 0.5f * wv * ss * ir;
+        if (HALF) rb += -W7 * ss / (2.f * rho * rho * nu);
+        else rb -= 0.5f * wv * ss * ir;
 #pragma unroll
         for (int e = 0; e < 6; ++e) {
             const float mult = (e < 3 ? 1.f : 2.f);  // off-diagonals appear twice
-            const float pb = kw * sig[e] * mult;
+            const float pb = HALF ? -k * W7 * sig[e] / (rho * nu) * mult : kw * sig[e] * mult;
             const int i0 = ia[e], i1 = ib[e];
             Sb[e] += pb;
             rb -= pb * ((e < 3 ? 1.f / 3.f : 0.f) + u[i0] * u[i1]);
@@ -1273,13 +1376,13 @@ __device__ __forceinline__ float response_vjp(float rp, const float (&u)[3], con
         ub[d] -= Fb[d] * rho * alpha;
     }
     const float s = 1.f + 0.5f * alpha;
-    const float inv_s = 1.f / s, inv = inv_s * ir;
+    const float inv_s = 1.f / s, inv = HALF ? 1.f / (s * rho) : inv_s * ir;
     float mb[3], sbar = 0.f;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         mb[d] = ub[d] * inv;
         rb -= ub[d] * (s * u[d] - 0.5f * P.a[d]) * inv;
-        sbar -= ub[d] * u[d] * inv_s;
+        sbar -= HALF ? ub[d] * u[d] / s : ub[d] * u[d] * inv_s;
     }
     abar += 0.5f * sbar;
 #pragma unroll

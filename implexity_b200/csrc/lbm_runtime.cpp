@@ -1800,14 +1800,19 @@ SeedParams stage_seed(const lbm_handle& h, const double* w, double scale) {
     return sp;
 }
 
-// The scales of the stored cotangent are powers of two: their quotients are
+// The scales of a stored FP32 cotangent are powers of two: their quotients are
 // exact, where a rounded one (1 +- 6e-8) enters every step of a segment alike
 // and made the whole horizon gradient too long by up to 3e-6 after 400 steps.
+// A 16-bit cotangent is scaled to a root mean square of one: nearly uniform
+// values then lie where the spacing of the format halves.  The nearest power of
+// two would put them anywhere between 0.7 and 1.4 (FP16 gradients of D3Q19 MRT
+// and D3Q27 horizons: 3.4e-4 and 2.0e-4 off FP64 instead of 1.3e-4 and 1.5e-4).
 float power_of_two(double v) {
     if (!(v > 0) || !std::isfinite(v)) return 1.f;
     const double p = std::exp2(std::round(std::log2(v)));
     return p >= 1e-37 && p <= 1e37 ? (float)p : 1.f;
 }
+bool exact_scales(const lbm_handle& h) { return h.lam_storage == LBM_STORE_F32; }
 
 double seed(lbm_handle& h, const double* w, AdjState& st, float* record, double stage_scale = 1.0) {
     int64_t* ctr = &h.device_bytes;
@@ -1828,7 +1833,9 @@ double seed(lbm_handle& h, const double* w, AdjState& st, float* record, double 
     CK(launch_objective(h.Q, h.storage, h.lam_storage, 1, a, grid_for(h), h.stream));
     const double n0 = read_norm(h);
     const double entries = (double)h.fluid_cells * h.Q;
-    st.s0 = n0 > 0 ? power_of_two(std::sqrt(entries) / n0) : 1.f;
+    const double unit = n0 > 0 ? std::sqrt(entries) / n0 : 1.0;
+    st.s0 = exact_scales(h) ? power_of_two(unit) : (float)unit;
+    if (!std::isfinite(st.s0) || st.s0 == 0.f) st.s0 = 1.f;
     st.scale = st.s0;
     st.target = st.s0;
     a.write_lambda = 1;
@@ -1854,6 +1861,7 @@ void alloc_adjoint(lbm_handle& h, int lam_storage) {
 float next_scale(const lbm_handle& h, double true_norm, float cur) {
     if (!(true_norm > 0) || !std::isfinite(true_norm)) return cur;
     double s = std::sqrt((double)h.fluid_cells * h.Q) / true_norm;
+    if (!exact_scales(h)) return std::isfinite(s) && s > 0 && s <= 3e38 ? (float)s : cur;
     if (!std::isfinite(s) || s < 1e-37 || s > 1e37) return cur;
     return power_of_two(s);
 }
