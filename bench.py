@@ -57,9 +57,9 @@ def launches(cells, T, storage, iterations):
     states, the forward passes, responses, two seeds, the transposed steps (residual checked every
     100) and two of the design-map transpose.  Staged forward passes are one launch each and one per
     16 for their partials; runs of steps (16-bit storage, or a small grid) one for as many passes as
-    8 MB of partials hold (128 at most) and one for the partials."""
+    12 MB of partials hold (128 at most) and one for the partials."""
     wide = storage == "float32"
-    run = min(128, max(8, (8 << 20) // (min(-(-cells // 256) * 8, 148 * 64) * 32)))
+    run = min(128, max(8, (12 << 20) // (min(-(-cells // 256) * 8, 148 * 64) * 48)))
     forward = T + 1 + -(-(T + 1) // 16) if wide and cells > 640 << 10 else 2 * -(-(T + 1) // run)
     adjoint = iterations if cells > (640 << 10 if wide else 900 << 10) else iterations / 100
     return 1 + 1 + 2 + forward + 1 + 2 + adjoint + 2

@@ -1518,11 +1518,47 @@ __device__ __forceinline__ float warp_max(float v) {
     asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
     return r;
 }
-// FP64 sum of per-thread FP32 partial sums.
-__device__ __forceinline__ double warp_sum(double v) {
+// Compensated sums of N (2 or 8) values over a warp: the lanes of each half
+// take over half of the values at a time, so that 5 (9) merges do what N trees
+// of five would.  Lane k * 32 / N then holds the sum of value k as h + l, the
+// rounding errors of h's additions being gathered in l (Neumaier's summation).
+__device__ __forceinline__ void gather_error(double& h, double& l, double oh, double ol) {
+    double s, e;
+    two_sum(h, oh, s, e);
+    h = s;
+    l += ol + e;
+}
+template <int N>
+__device__ __forceinline__ void warp_sums(const double (&v)[N], double& h, double& l) {
+    const int lane = threadIdx.x & 31;
+    double hs[N / 2], ls[N / 2];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(FULL, v, off);
-    return v;
+    for (int k = 0; k < N / 2; ++k) {  // the values are exact as yet
+        const bool up = lane & 16;
+        two_sum(up ? v[k + N / 2] : v[k], __shfl_xor_sync(FULL, up ? v[k] : v[k + N / 2], 16), hs[k], ls[k]);
+    }
+    int off = 8;
+#pragma unroll
+    for (int half = N / 4; half > 0; half /= 2, off /= 2) {
+        const bool up = lane & off;
+#pragma unroll
+        for (int k = 0; k < half; ++k) {
+            const double oh = __shfl_xor_sync(FULL, up ? hs[k] : hs[k + half], off);
+            const double ol = __shfl_xor_sync(FULL, up ? ls[k] : ls[k + half], off);
+            if (up) {
+                hs[k] = hs[k + half];
+                ls[k] = ls[k + half];
+            }
+            gather_error(hs[k], ls[k], oh, ol);
+        }
+    }
+#pragma unroll
+    for (; off > 0; off /= 2) {
+        const double oh = __shfl_xor_sync(FULL, hs[0], off), ol = __shfl_xor_sync(FULL, ls[0], off);
+        gather_error(hs[0], ls[0], oh, ol);
+    }
+    h = hs[0];
+    l = ls[0];
 }
 
 // A warp's share of a pass's admission record; k_reduce_partials combines the
@@ -1530,22 +1566,28 @@ __device__ __forceinline__ double warp_sum(double v) {
 // the blocks' partials: two FP64 block reductions and a fence, 3 to 4 us in
 // the tail of every step.)
 __device__ __forceinline__ void store_partial(const DiagLocal& acc, StepPartial* out) {
-    const double mass = warp_sum((double)acc.mass), exch = warp_sum((double)acc.exch);
+    const int lane = threadIdx.x & 31;
+    double h, l;
+    warp_sums<2>({(double)acc.mass, (double)acc.exch}, h, l);
     const float mn = warp_min(acc.minf), mx = warp_max(acc.maxu2);
     const bool nf = __any_sync(FULL, acc.nf);
-    if ((threadIdx.x & 31) == 0) {
-        out->mass = mass;
-        out->exch = exch;
+    if (lane % 16 == 0) {
+        out->sum[lane / 8] = h;
+        out->sum[lane / 8 + 1] = l;
+    }
+    if (lane == 0) {
         out->min_f = mn;
         out->max_u2 = mx;
         out->nonfinite = nf;
     }
 }
 __device__ __forceinline__ void store_response_partial(const double (&r)[8], double* out) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const double s = warp_sum(r[k]);
-        if ((threadIdx.x & 31) == 0) out[k] = s;
+    const int lane = threadIdx.x & 31;
+    double h, l;
+    warp_sums<8>(r, h, l);
+    if (lane % 4 == 0) {
+        out[lane / 2] = h;
+        out[lane / 2 + 1] = l;
     }
 }
 

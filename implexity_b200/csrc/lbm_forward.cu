@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(TPB, (Q == 19 ? 3 : 2)) k_forward(FwdArgs a) {
     if (warp > 0) {
         const uint32_t w = blockIdx.x * CONSUMER_WARPS + (uint32_t)(warp - 1);
         if (a.partial) store_partial(acc, a.partial + w);
-        if constexpr (RSP) store_response_partial(rsum, a.rpartial + (size_t)w * 8);
+        if constexpr (RSP) store_response_partial(rsum, a.rpartial + (size_t)w * RESPONSE_PARTIAL);
     }
 }
 

@@ -22,12 +22,14 @@ enum StoreKind { ST_F32 = 0, ST_F16 = 1, ST_BF16 = 2 };
 // the bulk moment of the Gram-Schmidt basis (b = |c|^2 - 1), folded at compile time
 enum CollKind { CK_PAIRS = 0, CK_MRT = 1, CK_MRT_BULK = 2 };
 
-// One warp's share of a pass's admission record.
+// One warp's share of a pass's admission record: compensated sums (high and
+// low parts) of the mass and the port exchange, extrema, flag.
 struct StepPartial {
-    double mass, exch;
+    double sum[4];
     float min_f, max_u2;
     int32_t nonfinite, pad;
 };
+constexpr int RESPONSE_PARTIAL = 16;  // doubles: eight compensated sums
 
 struct FwdArgs {
     Geometry G;
@@ -45,7 +47,7 @@ struct FwdArgs {
     int32_t bulk_store;      // full tiles leave through bulk stores (planes 16-byte aligned)
     uint32_t step;           // absolute step index (seeds the stochastic rounding)
     int* err;                // set when a bounded wait gave up
-    // response sums of the state the step reads, 8 per warp (nullptr: off)
+    // response sums of the state the step reads, RESPONSE_PARTIAL doubles per warp (nullptr: off)
     double* rpartial;
     const float* phi;        // design density (response 5)
     SeedParams sp;           // unit conversions of the responses (w unused)

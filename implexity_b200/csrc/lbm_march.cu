@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(MT, MB) k_march_forward(const __grid_constant_
         }
         // the pass's record, while the barrier fills
         if (a.partial) store_partial(acc, a.partial + (size_t)pass * warps + warp);
-        if constexpr (RSP) store_response_partial(rsum, a.rpartial + ((size_t)pass * warps + warp) * 8);
+        if constexpr (RSP) store_response_partial(rsum, a.rpartial + ((size_t)pass * warps + warp) * RESPONSE_PARTIAL);
         if (more) {
             if (threadIdx.x == 0) go = grid_wait(g.bar, (unsigned)(pass + 1) * gridDim.x, a.err);
             __syncthreads();
@@ -387,7 +387,7 @@ cudaError_t run_march(MarchFwdArgs& g, cudaStream_t s) {
         if (!g.a.G.periodic && three_blocks(g.a.G.n)) kernel = k_march_forward<Q, COLL, T, RSP, DP, 0, 3>;
     const MarchShape sh = march_shape(kernel, g.a.G.n);
     const uint32_t warps = (uint32_t)(sh.grid * sh.threads / 32);
-    const int64_t per_pass = (int64_t)warps * ((g.diag ? sizeof(StepPartial) : 0) + (RSP ? 64 : 0));
+    const int64_t per_pass = (int64_t)warps * ((g.diag ? sizeof(StepPartial) : 0) + (RSP ? RESPONSE_PARTIAL * sizeof(double) : 0));
     if (per_pass * g.n_pass > g.scratch_bytes) return cudaErrorInvalidValue;
     g.a.partial = g.diag ? static_cast<StepPartial*>(g.scratch) : nullptr;
     g.a.rpartial = RSP ? reinterpret_cast<double*>(static_cast<char*>(g.scratch) +
@@ -432,9 +432,14 @@ cudaError_t LBM_PART_NAME(march_adjoint)(int storage, MarchAdjArgs& g, cudaStrea
 }
 #else
 namespace {
-// One block per pass: the warps' partials combined in a fixed order.
-__global__ void __launch_bounds__(256) k_reduce_partials(const StepPartial* part, const double* rpart,
-                                                         uint32_t warps, uint32_t stride, StepDiag* out, double* stage) {
+// One block per pass: the warps' partials combined in a fixed order.  Eight
+// threads share a warp's response sums, one pair each: with a thread per warp
+// and its eight sums one after the other, 64^3 runs spent 2.4 of 17.3 us a step
+// here.
+constexpr int REDUCE_THREADS = 512;
+__global__ void __launch_bounds__(REDUCE_THREADS) k_reduce_partials(const StepPartial* part, const double* rpart,
+                                                                    uint32_t warps, uint32_t stride, StepDiag* out,
+                                                                    double* stage) {
     const size_t pass = blockIdx.x;
     if (out) {
         DiagAcc acc;
@@ -442,10 +447,10 @@ __global__ void __launch_bounds__(256) k_reduce_partials(const StepPartial* part
         for (uint32_t i = threadIdx.x; i < warps; i += blockDim.x) {
             const StepPartial& p = part[pass * stride + i];
             DiagAcc o;
-            o.mh = p.mass;
-            o.ml = 0.0;
-            o.eh = p.exch;
-            o.el = 0.0;
+            o.mh = p.sum[0];
+            o.ml = p.sum[1];
+            o.eh = p.sum[2];
+            o.el = p.sum[3];
             o.minf = p.min_f;
             o.maxu2 = p.max_u2;
             o.nf = p.nonfinite;
@@ -464,18 +469,28 @@ __global__ void __launch_bounds__(256) k_reduce_partials(const StepPartial* part
         }
     }
     if (stage) {
-        Sums<8> s;
-        s.init();
-        for (uint32_t i = threadIdx.x; i < warps; i += blockDim.x)
+        __shared__ double2 sums[REDUCE_THREADS / 32][8];
+        const uint32_t k = threadIdx.x & 7;
+        const double2* p = reinterpret_cast<const double2*>(rpart + pass * stride * RESPONSE_PARTIAL);
+        double h = 0.0, l = 0.0;
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x >> 3; i < warps; i += REDUCE_THREADS / 8) {
+            const double2 v = p[i * 8 + k];
+            dd_add(h, l, v.x, v.y);
+        }
 #pragma unroll
-            for (int k = 0; k < 8; ++k) s.add(k, rpart[(pass * stride + i) * 8 + k]);
-        s = block_reduce_sums<8>(s);
-        if (threadIdx.x == 0)
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                stage[pass * 16 + 2 * k] = s.h[k];
-                stage[pass * 16 + 2 * k + 1] = s.l[k];
-            }
+        for (int off = 8; off < 32; off *= 2) {
+            const double oh = __shfl_xor_sync(FULL, h, off), ol = __shfl_xor_sync(FULL, l, off);
+            dd_add(h, l, oh, ol);
+        }
+        if ((threadIdx.x & 31) < 8) sums[threadIdx.x >> 5][k] = make_double2(h, l);
+        __syncthreads();
+        if (threadIdx.x < 8) {
+            h = l = 0.0;
+            for (int w = 0; w < REDUCE_THREADS / 32; ++w) dd_add(h, l, sums[w][k].x, sums[w][k].y);
+            stage[pass * 16 + 2 * k] = h;
+            stage[pass * 16 + 2 * k + 1] = l;
+        }
     }
 }
 
@@ -486,12 +501,12 @@ int64_t pass_warps(int64_t n, int sms) {
     return std::min<int64_t>((n + 255) / 256 * 8, (int64_t)sms * 64);
 }
 int64_t march_scratch(int64_t n, int sms, bool stage) {
-    return pass_warps(n, sms) * (int64_t)(sizeof(StepPartial) + (stage ? 64 : 0));
+    return pass_warps(n, sms) * (int64_t)(sizeof(StepPartial) + (stage ? RESPONSE_PARTIAL * sizeof(double) : 0));
 }
 
 cudaError_t launch_reduce_partials(const StepPartial* part, const double* rpart, uint32_t warps, uint32_t stride,
                                    int passes, StepDiag* diag, double* stage, cudaStream_t s) {
-    k_reduce_partials<<<passes, 256, 0, s>>>(part, rpart, warps, stride, diag, stage);
+    k_reduce_partials<<<passes, REDUCE_THREADS, 0, s>>>(part, rpart, warps, stride, diag, stage);
     return cudaGetLastError();
 }
 

@@ -1217,7 +1217,7 @@ void staged_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* d
     const int64_t W = pass_warps(h.n(), h.sms), chunk = std::min<int64_t>(16, passes);
     DevBuf buf;
     if (diag || stage)
-        buf.alloc_pooled((size_t)(chunk * W) * (sizeof(StepPartial) + 64), &h.device_bytes, h.device, h.stream);
+        buf.alloc_pooled((size_t)(chunk * W) * (sizeof(StepPartial) + RESPONSE_PARTIAL * sizeof(double)), &h.device_bytes, h.device, h.stream);
     StepPartial* const part = buf.as<StepPartial>();
     double* const rpart = buf.p ? reinterpret_cast<double*>(part + chunk * W) : nullptr;
     for (int64_t i = 0; i < passes;) {
@@ -1225,7 +1225,7 @@ void staged_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* d
         uint32_t warps = 0;
         for (int64_t j = 0; j < k; ++j)
             pass(h, !(inspect_last && i + j == passes - 1), diag ? part + j * W : nullptr,
-                 stage ? rpart + j * W * 8 : nullptr, record ? record + (size_t)(i + j) * record_stride : nullptr,
+                 stage ? rpart + j * W * RESPONSE_PARTIAL : nullptr, record ? record + (size_t)(i + j) * record_stride : nullptr,
                  record_s, &warps);
         if (diag || stage)
             CK(launch_reduce_partials(part, rpart, warps, (uint32_t)W, (int)k, diag ? diag + i : nullptr,
@@ -1275,10 +1275,10 @@ bool marches(const lbm_handle& h, bool adjoint, bool stage) {
     return h.cooperative && h.n() <= most && coll_kernel(h) != CK_MRT && h.nee_groups.empty() && !h.slab;
 }
 
-// Passes of one launch: the partial records stay within 8 MB.
+// Passes of one launch: the partial records stay within 12 MB.
 int64_t march_chunk(lbm_handle& h, bool stage) {
     const int64_t per = march_scratch(h.n(), h.sms, stage);
-    return std::max<int64_t>(8, std::min<int64_t>(128, (8 << 20) / per));
+    return std::max<int64_t>(8, std::min<int64_t>(128, (12 << 20) / per));
 }
 
 // A run that does not fit the device as it is (another context holds part of
