@@ -328,112 +328,197 @@ void reconstruct(const HostLat& L, const PortSpec& p, const double a[3], const d
 }
 
 // ------------------------------------------------------------ device buffers
-// Handles' buffers and checkpoints come from one stream-ordered pool per
-// device.  With cudaMalloc / cudaFree on every gradient, the sixteen 320 MB
-// states of a horizon gradient cost 20 to 100 ms on a shared host, by the
-// neighbours' load.  Freed memory stays in the pool up to POOL_KEEP bytes, for
-// the next gradient or handle (the frees are ordered on the owner's stream, the
-// driver orders a reuse on another); a failing allocation gives it back first.
-constexpr uint64_t POOL_KEEP = 16ull << 30;
+// Handles' buffers, records and checkpoints are cudaMalloc's blocks that a list
+// keeps for the next gradient or handle when they are given back: with cudaMalloc
+// and cudaFree on every gradient, the sixteen 320 MB states of a horizon
+// gradient cost 20 to 100 ms on a shared host, by the neighbours' load.  (A
+// stream-ordered pool of the driver's maps memory in pages of 2 MB: 85 ms for
+// the 12.6 GB of a trajectory's records and as much to give them back, where
+// cudaMalloc takes 1 ms and cudaFree 6.)  A device's list holds IDLE_CAP bytes at
+// most, whatever its handles hold; what was given back first leaves first.  It
+// gives all back when an allocation fails and with the device's last handle.
+constexpr size_t IDLE_CAP = 16ull << 30;
 
-cudaMemPool_t state_pool(int device) {
-    static std::mutex mu;
-    static std::map<int, cudaMemPool_t> pools;
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = pools.find(device);
-    if (it != pools.end()) return it->second;
-    cudaMemPool_t pool = nullptr;
-    int ok = 0;
-    if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, device) == cudaSuccess && ok) {
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        uint64_t keep = POOL_KEEP;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
-            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)
-            pool = nullptr;
+struct Block {
+    void* p = nullptr;
+    size_t bytes = 0;
+    int device = 0;
+    cudaEvent_t last_use = nullptr;  // on the stream of the owner that gave it back
+};
+struct BlockList {
+    static constexpr size_t MOST = 256;  // idle blocks
+    std::mutex mu;
+    std::vector<Block> idle;         // the oldest first; never grows past MOST
+    std::map<int, int64_t> handles;  // of each device
+    BlockList() { idle.reserve(MOST); }
+};
+BlockList& block_list() {
+    static BlockList* list = new BlockList;  // not destroyed: handles may outlive static objects
+    return *list;
+}
+
+void destroy_block(const Block& b) {
+    cudaEventDestroy(b.last_use);
+    cudaFree(b.p);  // (waits for the device: a last use may be in flight)
+}
+// Frees a device's oldest idle blocks until `keep` bytes are left.
+void shrink_idle(BlockList& L, int device, size_t keep) {
+    size_t held = 0;
+    for (const Block& b : L.idle)
+        if (b.device == device) held += b.bytes;
+    for (size_t i = 0; i < L.idle.size() && held > keep;) {
+        if (L.idle[i].device != device) {
+            ++i;
+            continue;
+        }
+        held -= L.idle[i].bytes;
+        destroy_block(L.idle[i]);
+        L.idle.erase(L.idle.begin() + (std::ptrdiff_t)i);
+    }
+}
+void release_idle(int device) {
+    BlockList& L = block_list();
+    std::lock_guard<std::mutex> lock(L.mu);
+    shrink_idle(L, device, 0);
+}
+size_t idle_bytes(int device) {
+    BlockList& L = block_list();
+    std::lock_guard<std::mutex> lock(L.mu);
+    size_t held = 0;
+    for (const Block& b : L.idle)
+        if (b.device == device) held += b.bytes;
+    return held;
+}
+// cudaMalloc on the current device, with the idle blocks given back if it fails.
+cudaError_t device_malloc(void** p, size_t bytes, int device) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
+        release_idle(device);
+        e = cudaMalloc(p, bytes);
     }
-    return pools[device] = pool;
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+}
+// A block of at least `bytes` for work queued on stream s from now on.  An idle
+// one serves if it is not much larger: the rest of it would be lost.
+cudaError_t take_block(size_t bytes, int device, cudaStream_t s, Block* out) {
+    {
+        BlockList& L = block_list();
+        std::lock_guard<std::mutex> lock(L.mu);
+        size_t best = L.idle.size();
+        for (size_t i = 0; i < L.idle.size(); ++i) {
+            const Block& b = L.idle[i];
+            if (b.device == device && b.bytes >= bytes && b.bytes <= bytes + bytes / 4 + (64 << 10) &&
+                (best == L.idle.size() || b.bytes < L.idle[best].bytes))
+                best = i;
+        }
+        if (best < L.idle.size()) {
+            *out = L.idle[best];
+            L.idle.erase(L.idle.begin() + (std::ptrdiff_t)best);
+        }
+    }
+    cudaError_t e;
+    if (out->p) {
+        e = cudaStreamWaitEvent(s, out->last_use, 0);
+        if (e != cudaSuccess) destroy_block(*out);
+    } else {
+        e = device_malloc(&out->p, bytes, device);
+        out->bytes = bytes;
+        out->device = device;
+        if (e == cudaSuccess) {
+            e = cudaEventCreateWithFlags(&out->last_use, cudaEventDisableTiming);
+            if (e != cudaSuccess) cudaFree(out->p);
+        }
+    }
+    if (e != cudaSuccess) *out = Block{};
+    return e;
+}
+// Gives a block back after the work queued on s so far.
+void give_block(const Block& b, cudaStream_t s) {
+    if (cudaEventRecord(b.last_use, s) != cudaSuccess) {
+        cudaGetLastError();
+        destroy_block(b);
+        return;
+    }
+    BlockList& L = block_list();
+    std::lock_guard<std::mutex> lock(L.mu);
+    if (L.idle.size() == BlockList::MOST) {
+        destroy_block(L.idle.front());
+        L.idle.erase(L.idle.begin());
+    }
+    L.idle.push_back(b);
+    shrink_idle(L, b.device, IDLE_CAP);
 }
 
-// Gives the pool's unused memory back to the device.
-void trim_pool() {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return;
-    if (cudaMemPool_t pool = state_pool(dev)) {
-        cudaDeviceSynchronize();  // pending frees reach the pool
-        cudaMemPoolTrimTo(pool, 0);
+// A handle's place among those of its device: the idle blocks go with the last
+// one, for other allocators and processes.
+struct Presence {
+    int device = -1;
+    Presence() = default;
+    Presence(const Presence&) = delete;
+    Presence& operator=(const Presence&) = delete;
+    void enter(int dev) {
+        BlockList& L = block_list();
+        std::lock_guard<std::mutex> lock(L.mu);
+        ++L.handles[dev];
+        device = dev;
     }
-}
-
-// Bytes the pool holds and nobody uses.
-size_t pool_idle(int device) {
-    uint64_t held = 0, used = 0;
-    cudaMemPool_t pool = state_pool(device);
-    if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
-        return 0;
-    return held > used ? (size_t)(held - used) : 0;
-}
+    ~Presence() {
+        if (device < 0) return;
+        BlockList& L = block_list();
+        std::lock_guard<std::mutex> lock(L.mu);
+        if (--L.handles[device] == 0) shrink_idle(L, device, 0);
+    }
+};
 
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
     int64_t* counter = nullptr;
-    cudaStream_t pooled = nullptr;  // the stream that frees a buffer of the pool
+    Block block;                     // of the list (block.p set), given back in
+    cudaStream_t stream = nullptr;   // the order of this stream
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { reset(); }
     void reset() {
         if (p) {
-            if (pooled) cudaFreeAsync(p, pooled);
+            if (block.p) give_block(block, stream);
             else cudaFree(p);
             if (counter) *counter -= (int64_t)bytes;
         }
         p = nullptr;
-        pooled = nullptr;
+        block = Block{};
         bytes = 0;
     }
     void alloc(size_t b, int64_t* ctr) {
         if (p && bytes >= b) return;
         reset();
-        counter = ctr;
-        cudaError_t e = cudaMalloc(&p, b);
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            trim_pool();
-            e = cudaMalloc(&p, b);
-        }
-        if (e != cudaSuccess) p = nullptr;
-        CK(e);
-        bytes = b;
-        if (counter) *counter += (int64_t)b;
+        int device = 0;
+        CK(cudaGetDevice(&device));
+        CK(device_malloc(&p, b, device));
+        count(b, ctr);
     }
-    // b bytes of the device's pool, used and freed in the order of stream s
+    // b bytes of the device's list, used and given back in the order of stream s
     void alloc_pooled(size_t b, int64_t* ctr, int device, cudaStream_t s) {
         reset();
-        if (cudaMemPool_t pool = state_pool(device)) {
-            if (cudaMallocFromPoolAsync(&p, b, pool, s) == cudaSuccess) {
-                pooled = s;
-                bytes = b;
-                counter = ctr;
-                if (counter) *counter += (int64_t)b;
-                return;
-            }
-            cudaGetLastError();
-            p = nullptr;
-        }
-        alloc(b, ctr);
+        CK(take_block(b, device, s, &block));
+        p = block.p;
+        stream = s;
+        count(b, ctr);
     }
-    // at least b bytes of the pool: the buffers of a handle's first gradient or
+    void count(size_t b, int64_t* ctr) {
+        bytes = b;
+        counter = ctr;
+        if (counter) *counter += (int64_t)b;
+    }
+    // at least b bytes of the list: the buffers of a handle's first gradient or
     // read-back, which a new handle then takes from an old one
     void grow(size_t b, int64_t* ctr, int device, cudaStream_t s) {
         if (!p || bytes < b) alloc_pooled(b, ctr, device, s);
     }
-    // exactly b bytes of the pool (releases a larger buffer)
+    // exactly b bytes of the list (gives another size back)
     void fit(size_t b, int64_t* ctr, int device, cudaStream_t s) {
         if (!p || bytes != b) alloc_pooled(b, ctr, device, s);
     }
@@ -565,6 +650,7 @@ struct AdjState;
 }  // namespace
 
 struct lbm_handle {
+    Presence presence;  // the first member: it leaves after every buffer
     lbm_handle() { pin_handles(1); }
     ~lbm_handle() { pin_handles(-1); }
     // --- normalised problem
@@ -1102,6 +1188,7 @@ void validate_and_build(lbm_handle& h, const lbm_problem_t& p) {
 
     // --- device
     CK(cudaGetDevice(&h.device));
+    h.presence.enter(h.device);
     CK(cudaDeviceGetAttribute(&h.sms, cudaDevAttrMultiProcessorCount, h.device));
     int coop = 0;
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h.device));
@@ -1217,7 +1304,8 @@ void staged_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* d
     const int64_t W = pass_warps(h.n(), h.sms), chunk = std::min<int64_t>(16, passes);
     DevBuf buf;
     if (diag || stage)
-        buf.alloc_pooled((size_t)(chunk * W) * (sizeof(StepPartial) + RESPONSE_PARTIAL * sizeof(double)), &h.device_bytes, h.device, h.stream);
+        buf.alloc_pooled((size_t)(chunk * W) * (sizeof(StepPartial) + RESPONSE_PARTIAL * sizeof(double)),
+                         &h.device_bytes, h.device, h.stream);
     StepPartial* const part = buf.as<StepPartial>();
     double* const rpart = buf.p ? reinterpret_cast<double*>(part + chunk * W) : nullptr;
     for (int64_t i = 0; i < passes;) {
@@ -1572,14 +1660,14 @@ DesignArgs design_args(lbm_handle& h) {
 // IO_CAP bytes; with `unit` a value outside [0, 1] sets the handle's flag.
 constexpr int64_t IO_CAP = 64 << 20;
 
-// (from the pool: a new handle's first call allocates nothing)
+// (from the list: a new handle's first call allocates nothing)
 void io_buffer(lbm_handle& h, DevBuf& io, int64_t values) {
     io.alloc_pooled((size_t)std::min<int64_t>(values * 8, IO_CAP), &h.device_bytes, h.device, h.stream);
 }
 
 //
 // Up to HOST_VALUES values the host converts and checks: fewer calls than the
-// pool, the kernel and the flag take (set_design of 1280 cells 50 -> 33 us).
+// list, the kernel and the flag take (set_design of 1280 cells 50 -> 33 us).
 // Returns false for a value outside [0, 1] seen there.
 constexpr int64_t HOST_VALUES = 16 << 10;
 
@@ -1958,7 +2046,7 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
     const size_t rec_stride = ((size_t)h.n() * rec_planes + 3) / 4 * 4;
     const size_t rec_bytes = rec_stride * sizeof(float);
     // With the checkpoint interval left to the library, the records of the
-    // whole trajectory are kept where the pool can keep them too (and half of
+    // whole trajectory are kept where the list can keep them too (and half of
     // what is free): the forward sweep writes them as it goes and
     // nothing is recomputed, which is a quarter to a third of the gradient
     // (256x128x128 MRT, 200 steps: 90.5 -> 64 ms; 48x24x24, 800 steps: 10.7 -> 7
@@ -1974,11 +2062,11 @@ lbm_status gradient_horizon(lbm_handle& h, const double* w, const lbm_adjoint_op
     {
         size_t free_b = 0, total_b = 0;
         CK(cudaMemGetInfo(&free_b, &total_b));
-        // the memory left, with what the pool keeps and the record of the last call
-        free_b += pool_idle(h.device) + h.record.bytes;
+        // the memory left, with the list's and the record of the last call
+        free_b += idle_bytes(h.device) + h.record.bytes;
         const size_t ab = h.array_bytes(h.storage);
         const size_t all = (size_t)(T + 1) * rec_bytes + CELL_PAD * sizeof(float);
-        if (o.checkpoint_every <= 0 && o.record_budget_bytes <= 0 && all <= std::min<size_t>(POOL_KEEP, free_b / 2)) {
+        if (o.checkpoint_every <= 0 && o.record_budget_bytes <= 0 && all <= std::min<size_t>(IDLE_CAP, free_b / 2)) {
             try {
                 whole.alloc_pooled(all, ctr, h.device, h.stream);
             } catch (const CudaError&) {  // taken by someone else meanwhile: checkpoints instead
@@ -2399,7 +2487,7 @@ void lbm_destroy(lbm_handle* h) {
     h->slab_adj = nullptr;
     if (h->stream) cudaStreamSynchronize(h->stream);
     h->ckpts.clear();
-    // the pool's buffers go back in the order of the stream, before it goes
+    // the list's blocks go back in the order of the stream, before it goes
     for (DevBuf* b : {&h->pop, &h->mask, &h->alpha, &h->phi, &h->raw, &h->den, &h->slope, &h->cls_d, &h->fixed_d,
                       &h->offsets_d, &h->ports_d, &h->partial, &h->counter, &h->sums, &h->errflag, &h->nee_cells_d,
                       &h->lam, &h->record, &h->abar, &h->abar_final, &h->phibar, &h->scale, &h->grad, &h->scratch,
