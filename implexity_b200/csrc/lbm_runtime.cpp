@@ -17,12 +17,11 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "../../include/lbm_b200.h"
 #include "lbm_common.cuh"
+#include "lbm_host.h"
 #include "lbm_launch.h"
 #include "lbm_revolve.h"
 
@@ -538,8 +537,9 @@ constexpr int64_t PIN_CAP = 32 << 20;
 
 struct PinList {
     std::mutex mu;
-    std::vector<std::pair<void*, size_t>> idle;
+    std::vector<std::pair<void*, size_t>> idle;  // never grows past its reserve: a lease ends without allocating
     int64_t handles = 0;
+    PinList() { idle.reserve(8); }
 };
 PinList& pin_list() {
     static PinList* list = new PinList;  // not destroyed: handles may outlive static objects
@@ -602,38 +602,6 @@ struct PinLease {
     float* floats() const { return static_cast<float*>(p); }
 };
 size_t pin_bytes(int64_t values) { return (size_t)std::min<int64_t>(values * 4, PIN_CAP); }
-
-// fn(begin, end) over [0, n), in chunks that helper threads share with the
-// calling one where the work is worth it.  The caller takes chunks itself and
-// waits only for chunks in progress: a helper that is not scheduled in time
-// (the caller's own thread pool may still spin on every core) finds nothing
-// left and leaves without touching fn.
-template <typename F>
-void parallel_range(int64_t n, F&& fn) {
-    constexpr int64_t CHUNK = 1 << 16;
-    struct Job {
-        std::atomic<int64_t> next{0}, done{0};
-    };
-    const int64_t chunks = (n + CHUNK - 1) / CHUNK;
-    const auto take = [n, chunks](Job& job, F& f) {
-        for (int64_t c; (c = job.next.fetch_add(1)) < chunks; job.done.fetch_add(1)) f(c * CHUNK, std::min(n, (c + 1) * CHUNK));
-    };
-    if (chunks < 4) {
-        if (n > 0) fn((int64_t)0, n);
-        return;
-    }
-    const auto job = std::make_shared<Job>();
-    const int64_t helpers = std::min<int64_t>({7, (int64_t)std::thread::hardware_concurrency() - 1, chunks / 2 - 1});
-    for (int64_t k = 0; k < helpers; ++k) {
-        try {
-            std::thread([job, take, &fn] { take(*job, fn); }).detach();
-        } catch (const std::system_error&) {  // no more threads
-            break;
-        }
-    }
-    take(*job, fn);
-    while (job->done.load() < chunks) std::this_thread::yield();
-}
 
 size_t storage_bytes(int s) { return s == LBM_STORE_F32 ? 4 : 2; }
 
