@@ -24,7 +24,7 @@ enum CollKind { CK_PAIRS = 0, CK_MRT = 1, CK_MRT_BULK = 2 };
 
 // One warp's share of a pass's admission record: compensated sums (high and
 // low parts) of the mass and the port exchange, extrema, flag.
-struct StepPartial {
+struct alignas(16) StepPartial {
     double sum[4];
     float min_f, max_u2;
     int32_t nonfinite, pad;

@@ -444,16 +444,19 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_reduce_partials(const StepPa
     if (out) {
         DiagAcc acc;
         acc.init();
-        for (uint32_t i = threadIdx.x; i < warps; i += blockDim.x) {
-            const StepPartial& p = part[pass * stride + i];
+        const double2* const p = reinterpret_cast<const double2*>(part + pass * stride);
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < warps; i += REDUCE_THREADS) {
+            const double2 mass = p[3 * i], exch = p[3 * i + 1];
+            const int4 rest = reinterpret_cast<const int4*>(p)[3 * i + 2];
             DiagAcc o;
-            o.mh = p.sum[0];
-            o.ml = p.sum[1];
-            o.eh = p.sum[2];
-            o.el = p.sum[3];
-            o.minf = p.min_f;
-            o.maxu2 = p.max_u2;
-            o.nf = p.nonfinite;
+            o.mh = mass.x;
+            o.ml = mass.y;
+            o.eh = exch.x;
+            o.el = exch.y;
+            o.minf = __int_as_float(rest.x);
+            o.maxu2 = __int_as_float(rest.y);
+            o.nf = rest.z;
             acc.merge(o);
         }
         acc = block_reduce(acc);

@@ -647,6 +647,7 @@ struct lbm_handle {
     DevBuf pop, mask, alpha, phi, raw, den, slope, cls_d, fixed_d, offsets_d, ports_d, partial, counter, diag;
     DevBuf lam, record, abar, abar_final, phibar, scale, grad, norm2, sums, scratch, errflag;
     DevBuf omega_cell, tau_state, tau_bar;
+    DevBuf pass_parts;  // partial admission records and response sums of a run of passes
     AdjState* slab_adj = nullptr;  // x-slab steady adjoint in progress (lbm_slab_adjoint_begin)
     int lam_storage = LBM_STORE_F32;
     // --- ports: normalised specs with their signals; pulsatile ports keep one
@@ -1264,18 +1265,25 @@ void pass(lbm_handle& h, bool collide, StepPartial* partial, double* rpartial, f
     ++h.t;
 }
 
+// Memory for the passes' partial records, kept by the handle: a step on its own
+// (a slab's, an extrapolating port's) takes none from the list and gives none back.
+void* pass_partials(lbm_handle& h, int64_t bytes) {
+    h.pass_parts.grow((size_t)bytes, &h.device_bytes, h.device, h.stream);
+    return h.pass_parts.p;
+}
+
 // `passes` passes launched one by one; with inspect_last the last one is
 // load-only.  diag / record / stage point at the first pass's slots (stage: 16
 // doubles per pass).  The partials of up to 16 passes are combined at once.
 void staged_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* diag, float* record,
                    int64_t record_stride, bool record_s, double* stage) {
     const int64_t W = pass_warps(h.n(), h.sms), chunk = std::min<int64_t>(16, passes);
-    DevBuf buf;
-    if (diag || stage)
-        buf.alloc_pooled((size_t)(chunk * W) * (sizeof(StepPartial) + RESPONSE_PARTIAL * sizeof(double)),
-                         &h.device_bytes, h.device, h.stream);
-    StepPartial* const part = buf.as<StepPartial>();
-    double* const rpart = buf.p ? reinterpret_cast<double*>(part + chunk * W) : nullptr;
+    StepPartial* part = nullptr;
+    double* rpart = nullptr;
+    if (diag || stage) {
+        part = static_cast<StepPartial*>(pass_partials(h, chunk * march_scratch(h.n(), h.sms, stage != nullptr)));
+        rpart = reinterpret_cast<double*>(part + chunk * W);
+    }
     for (int64_t i = 0; i < passes;) {
         const int64_t k = std::min(chunk, passes - i);
         uint32_t warps = 0;
@@ -1361,8 +1369,7 @@ void run_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* diag
     ensure_port_maps(h, h.t + passes);
     const int64_t chunk = march_chunk(h, stage != nullptr);
     const int64_t scratch = chunk * march_scratch(h.n(), h.sms, stage != nullptr);
-    DevBuf partial;  // the passes' partial records
-    if (diag || stage) partial.alloc_pooled((size_t)scratch, &h.device_bytes, h.device, h.stream);
+    void* const partial = diag || stage ? pass_partials(h, scratch) : nullptr;
     for (int64_t i = 0; i < passes;) {
         const int64_t k = std::min(chunk, passes - i);
         const bool inspects = inspect_last && i + k == passes;
@@ -1381,7 +1388,7 @@ void run_passes(lbm_handle& h, int64_t passes, bool inspect_last, StepDiag* diag
         g.record_stride = record_stride;
         g.diag = diag ? diag + i : nullptr;
         g.bar = reinterpret_cast<unsigned*>(h.word(2));
-        g.scratch = partial.p;
+        g.scratch = partial;
         g.scratch_bytes = scratch;
         if (!launched(h, launch_march_forward(h.Q, coll_kernel(h), h.storage, g, h.stream))) {
             run_passes(h, passes - i, inspect_last, g.diag, g.a.record, record_stride, record_s, g.stage);
@@ -2459,7 +2466,7 @@ void lbm_destroy(lbm_handle* h) {
     for (DevBuf* b : {&h->pop, &h->mask, &h->alpha, &h->phi, &h->raw, &h->den, &h->slope, &h->cls_d, &h->fixed_d,
                       &h->offsets_d, &h->ports_d, &h->partial, &h->counter, &h->sums, &h->errflag, &h->nee_cells_d,
                       &h->lam, &h->record, &h->abar, &h->abar_final, &h->phibar, &h->scale, &h->grad, &h->scratch,
-                      &h->diag, &h->tsums})
+                      &h->diag, &h->tsums, &h->pass_parts})
         b->reset();
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
@@ -3028,8 +3035,7 @@ int halo_dirs(const lbm_handle& h, int kind, int side, int32_t* dirs) {
 void read_slab_diag(lbm_handle& h, lbm_slab_diag_t* out) {
     StepDiag d{};
     CK(cudaMemcpyAsync(&d, h.diag.p, sizeof(d), cudaMemcpyDeviceToHost, h.stream));
-    CK(cudaStreamSynchronize(h.stream));
-    check_errflag(h);
+    check_errflag(h);  // (waits for the copy too)
     if (out) {
         out->mass = (double)h.fluid_cells + d.mass_hi + d.mass_lo;
         out->exchange = d.exch_hi + d.exch_lo;
