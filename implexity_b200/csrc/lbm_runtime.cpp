@@ -795,7 +795,10 @@ void ensure_port_maps(lbm_handle& h, int64_t t_max) {
     CK(cudaStreamSynchronize(h.stream));
     h.ports_d.reset();
     h.ports_d.alloc(h.maps_host.size() * sizeof(PortMap), &h.device_bytes);
-    CK(cudaMemcpy(h.ports_d.p, h.maps_host.data(), h.maps_host.size() * sizeof(PortMap), cudaMemcpyHostToDevice));
+    // on the handle's stream: a plain copy from pageable memory may return before
+    // its last bytes have landed, and this stream does not wait for the default one
+    CK(cudaMemcpyAsync(h.ports_d.p, h.maps_host.data(), h.maps_host.size() * sizeof(PortMap), cudaMemcpyHostToDevice,
+                       h.stream));
     h.map_states = states;
 }
 
@@ -2996,14 +2999,17 @@ lbm_status lbm_create_slab(const lbm_problem_t* problem, int32_t x_begin, int32_
         validate_and_build(*h, L);
         // ghost planes hold exchanged values and are never stepped
         std::vector<uint32_t> mask((size_t)nl);
-        CK(cudaMemcpy(mask.data(), h->mask.p, (size_t)nl * 4, cudaMemcpyDeviceToHost));
+        CK(cudaMemcpyAsync(mask.data(), h->mask.p, (size_t)nl * 4, cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
         int64_t fluid_own = 0;
         for (int64_t x = 0; x < nl; ++x) {
             const int64_t pl = x / sx;
             if (pl < hl || pl >= hl + own) mask[x] |= MASK_SOLID;
             else fluid_own += solid[x] ? 0 : 1;
         }
-        CK(cudaMemcpy(h->mask.p, mask.data(), (size_t)nl * 4, cudaMemcpyHostToDevice));
+        // (on the handle's stream, which does not wait for the default one)
+        CK(cudaMemcpyAsync(h->mask.p, mask.data(), (size_t)nl * 4, cudaMemcpyHostToDevice, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
         h->fluid_cells = fluid_own;
         g_create_error.clear();
         *out = h.release();
