@@ -37,7 +37,8 @@ struct AdjStage {
 // alpha cotangent ab_prev): the general path.
 template <int Q, int COLL, typename T, int AL, int STG, typename S>
 __device__ __forceinline__ void adj_one_cell(const AdjArgs& a, const S* st, int c, uint32_t x, uint32_t m, float ab_prev,
-                                             bool zwall, bool zlow, const T (&own)[ZWall<Q>::N], const T* B, T* D, uint32_t n, float s_in, float k_out, double& nsum) {
+                                             bool zwall, bool zlow, const T (&own)[ZWall<Q>::N], const T* B, T* D,
+                                             uint32_t n, float s_in, float k_out, double& nsum) {
     const bool fluid = !(m & MASK_SOLID);
     if (!fluid) return;
     float v[Q];
@@ -122,11 +123,12 @@ __device__ __forceinline__ void adj_one_cell(const AdjArgs& a, const S* st, int 
 // the recorded state as well and adds the state's response VJP.
 // Residency: 16-bit storage runs three blocks per SM (72 registers): its step
 // is bound by latency and instruction issue, not bytes, and a third block's
-// warps hide more of it (us per step with two / three, FP16: 256x128x128 114.0 /
-// 101.5, 128^3 63.6 / 52.9, D3Q27 192x128x128 120.1 / 109.3, with the registers
-// spilled).  FP32 storage keeps two (135.1 / 135.9, 71.6 / 72.4).
+// warps hide more of it (us per step with two / three, FP16: 256x128x128 126.3 /
+// 109.4, 128^3 69.7 / 57.2, D3Q27 192x128x128 128.4 / 113.9, with the registers
+// spilled).  The seeded D3Q27 step spills too much for it (250 / 258), and FP32
+// storage keeps two (135.1 / 135.9, 71.6 / 72.4).
 template <int Q, int COLL, typename T, int AL, int STG>
-__global__ void __launch_bounds__(TPB, (sizeof(T) == 2 ? 3 : 2)) k_adjoint(AdjArgs a) {
+__global__ void __launch_bounds__(TPB, (sizeof(T) == 2 && !(STG && Q == 27) ? 3 : 2)) k_adjoint(AdjArgs a) {
     constexpr int NREC = STG ? 10 : 4;
     using S = AdjStage<Q, T, NREC>;
     constexpr int NCOPY = Q + NREC + 2;  // runs of lambda, the record, mask and alpha
@@ -185,10 +187,12 @@ __global__ void __launch_bounds__(TPB, (sizeof(T) == 2 ? 3 : 2)) k_adjoint(AdjAr
         const float s_in = 1.f / a.in_scale_inv;        // stored scale of the input
         const float k_out = a.out_scale * a.in_scale_inv;  // stored input -> stored output
         using Z = ZWall<Q>;
-        // FP16 256x128x128: 106.0 -> 101.9 us per step.  FP32 storage is bound by
-        // bandwidth and gains nothing (D3Q27 lost 10% to the registers), nor does
-        // the forward step, whose registers then spill (124 -> 135 us).
-        constexpr bool PREFETCH = sizeof(T) == 2;
+        // FP16 256x128x128: 114.0 -> 109.4 us per step, D3Q27 192x128x128 148 -> 114,
+        // with stage seeds 277 -> 250; the seeded D3Q19 step at three blocks per SM
+        // has no registers to spare (263 -> 267).  FP32 storage is bound by bandwidth
+        // and gains nothing (D3Q27 lost 10% to the registers), nor does the forward
+        // step, whose registers then spill (124 -> 135 us).
+        constexpr bool PREFETCH = sizeof(T) == 2 && !(STG && Q == 19);
         ZWalk z(a.G, blockIdx.x * TILE + c0, gridDim.x * TILE);
         for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, z.next()) {
             const uint32_t x = tile * TILE + c0;
