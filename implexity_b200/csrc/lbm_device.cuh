@@ -1305,7 +1305,7 @@ __device__ __forceinline__ void second_moments(const float (&g)[Q], float (&S)[6
 // moments, so the adjoint step can seed a state from its record alone.
 // HALF: the seed enters a cotangent stored in 16 bits, whose trajectories keep
 // their order of operations (collide_vjp), a dozen divisions per cell and all
-// (267 us per seeded FP16 step of 256x128x128 cells, 161 without them).
+// (263 us per seeded FP16 step of 256x128x128 cells, 161 without them).
 template <int Q, bool HALF>
 __device__ __forceinline__ float response_vjp(float rp, const float (&u)[3], const float (&S)[6], float alpha,
                                               float dpw, bool port, const SeedParams& sp, const Physics& P,
@@ -1450,8 +1450,8 @@ __device__ __forceinline__ void dd_add(double& h, double& l, double h2, double l
 }
 
 // Per-thread admission accumulators (a thread sees a few tens of cells, so
-// single precision partial sums are exact to ~1e-7 of their own size; the
-// block and grid reductions are compensated double).
+// single precision partial sums are exact to ~1e-7 of their own size; the sums
+// over lanes, warps and blocks are compensated double).
 struct DiagLocal {
     float mass, exch, minf, maxu2;
     int nf;

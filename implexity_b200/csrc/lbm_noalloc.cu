@@ -7,11 +7,10 @@
 // front.  They already hold
 // their populations on the device and only want the numbers the admission
 // check of LbmProblem::admit (solver.rs:708-793) computes for one state.
-// The reduction here is the same one the stepping kernels run every step
-// (per-block compensated partials, then the last block combines them), but
-// its scratch is a file-scope static __device__ array instead of memory from
-// an lbm_handle: every GPU that loads the library holds it until the process
-// exits.
+// The sums are compensated as the stepping kernels' are: blocks leave their
+// partials and the last one combines them.  The scratch is a file-scope static
+// __device__ array instead of memory from an lbm_handle: every GPU that loads
+// the library holds it until the process exits.
 #include <algorithm>
 #include <cmath>
 #include <mutex>

@@ -1181,8 +1181,8 @@ void validate_and_build(lbm_handle& h, const lbm_problem_t& p) {
     h.fixed_d.grow((size_t)n * 4, ctr, h.device, h.stream);
     h.offsets_d.grow(std::max<size_t>(1, h.offsets.size()) * sizeof(int4), ctr, h.device, h.stream);
     h.ports_d.grow(std::max<size_t>(1, maps.size()) * sizeof(PortMap), ctr, h.device, h.stream);
-    h.partial.grow((size_t)h.sms * 32 * 16 * sizeof(double), ctr, h.device, h.stream);
-    h.counter.grow(2 * sizeof(unsigned), ctr, h.device, h.stream);  // [0] step/objective sums, [1] fused response sums
+    h.partial.grow((size_t)h.sms * 16 * 16 * sizeof(double), ctr, h.device, h.stream);  // eight sums of a block
+    h.counter.grow(sizeof(unsigned), ctr, h.device, h.stream);
     h.sums.grow(64 * sizeof(double), ctr, h.device, h.stream);
     CK(cudaMemsetAsync(h.mask.p, 0xff, (size_t)(n + CELL_PAD) * 4, h.stream));  // padding reads as solid
     CK(cudaMemcpyAsync(h.mask.p, mask.data(), (size_t)n * 4, cudaMemcpyHostToDevice, h.stream));
@@ -1200,7 +1200,7 @@ void validate_and_build(lbm_handle& h, const lbm_problem_t& p) {
     if (!maps.empty())
         CK(cudaMemcpyAsync(h.ports_d.p, maps.data(), maps.size() * sizeof(PortMap), cudaMemcpyHostToDevice,
                            h.stream));
-    CK(cudaMemsetAsync(h.counter.p, 0, 2 * sizeof(unsigned), h.stream));
+    CK(cudaMemsetAsync(h.counter.p, 0, sizeof(unsigned), h.stream));
     CK(cudaMemsetAsync(h.errflag.p, 0, h.errflag.bytes, h.stream));
     CK(cudaMemsetAsync(h.pop.p, 0, h.pop.bytes, h.stream));
     CK(cudaStreamSynchronize(h.stream));
@@ -1315,23 +1315,27 @@ void inspect(lbm_handle& h, StepDiag* diag, float* record, bool record_s = false
 // small enough for it to win and nothing runs between two steps: not for
 // extrapolating ports (a second kernel moves their cotangents after every
 // step), the general MRT collision or x-slabs (halos).
-// The limits, us per step of the staged kernels / of a run (B200):
-//   cells                       27 648      262 144      614 400      805 376    1 032 192   2 097 152   4 194 304
-//   forward FP32            8.7 / 3.4   12.9 / 9.4  23.1 / 21.4  29.6 / 33.0
-//   forward FP16            9.6 / 3.4   14.9 / 9.7  21.1 / 18.0  27.4 / 22.0  33.6 / 29.1  59.6 / 57.0   114 / 108
-//   forward D3Q27 FP32     12.7 / 4.5  19.3 / 12.9  40.5 / 35.3  44.0 / 43.1  53.7 / 53.7  95.5 / 103
-//   forward D3Q27 FP16     13.2 / 4.5  21.0 / 12.7  37.5 / 24.7  43.3 / 32.2  52.0 / 41.8  96.6 / 79.8   182 / 151
-//   forward FP64 collision 12.3 / 4.7  21.6 / 14.9  39.5 / 35.0  52.5 / 45.1  66.0 / 56.5   110 / 107
-//   adjoint FP32            8.3 / 3.1   14.2 / 9.0  24.9 / 23.9  30.6 / 33.7
-//   adjoint FP16            8.3 / 3.2   12.4 / 9.2  20.6 / 17.4  24.7 / 21.9  32.5 / 35.5
-//   adjoint D3Q27          10.3 / 4.0  18.5 / 12.2  40.1 / 34.6  43.8 / 42.6  54.1 / 53.3  99.2 / 103
-//   adjoint D3Q27 FP16     12.4 / 4.1  20.6 / 12.4  34.5 / 25.5  40.7 / 35.6  47.3 / 44.7  84.2 / 86.0
-// (the last before a third block per SM took 8% off its staged step)
-// and with the response sums 20.0 / 15.4 (262 144, FP32), 33.7 / 36.3 (614 400),
-// D3Q27 53.4 / 45.9 and 68.0 / 67.7 (1 032 192); with the stage seeds (a dozen
-// divisions per cell then) 24.0 / 22.9 and 47.4 / 52.6, D3Q27 30.2 / 26.2 and
-// 58.2 / 61.6.  The direct loads of a run
-// cost a 16-bit step less than the staged ring does, at every size measured.
+// The limits, us per step of the staged kernels / of a run (B200, one tree):
+//   cells                       27 648      262 144      614 400      811 668    1 032 192    2 097 152    4 194 304
+//   forward FP32             8.8 / 3.2  13.1 / 10.0  23.3 / 21.8  29.8 / 33.2  37.8 / 41.8  62.6 / 70.2
+//   forward FP16            10.6 / 3.4  15.2 / 10.1  21.5 / 18.5  27.1 / 22.1  33.9 / 31.0  60.0 / 57.6    115 / 110
+//   forward D3Q27 FP32      12.9 / 4.6  19.3 / 13.7  42.3 / 36.3  48.0 / 45.5  53.7 / 54.7  95.8 / 104
+//   forward D3Q27 FP16      13.0 / 4.7  20.9 / 13.2  37.8 / 25.5  40.0 / 31.7  56.2 / 42.6  98.4 / 81.5    183 / 155
+//   forward FP64 collision  10.8 / 3.8  19.3 / 12.0  32.0 / 28.4  42.5 / 37.5  54.4 / 46.8  89.9 / 90.1    166 / 173
+//   adjoint FP32             8.3 / 3.1   13.5 / 9.6  26.2 / 24.3  30.9 / 34.5  39.6 / 42.8
+//   adjoint FP16             8.3 / 3.4  12.5 / 10.2  22.7 / 20.6  26.8 / 23.7  33.1 / 38.0
+//   adjoint D3Q27 FP32      10.4 / 4.1  18.6 / 12.8  41.3 / 35.0  44.4 / 44.0  54.9 / 53.6  99.6 / 104
+//   adjoint D3Q27 FP16      14.5 / 4.3  20.5 / 13.3  32.9 / 27.4  39.6 / 36.2  52.0 / 46.9  82.5 / 90.3
+//   with response sums      11.3 / 5.8  20.5 / 15.2  33.5 / 35.4  43.3 / 44.9  53.8 / 55.1  88.9 / 104
+//     FP16                  11.6 / 5.9  20.2 / 16.4  29.2 / 29.0  38.3 / 33.3  46.1 / 47.8  86.3 / 98.2
+//     D3Q27                 15.2 / 7.1  26.7 / 19.2  52.4 / 46.5  56.8 / 55.3  66.0 / 67.9   119 / 128
+//     D3Q27 FP16            16.4 / 7.3  26.6 / 20.1  47.9 / 38.1  53.8 / 46.7  71.3 / 62.3   133 / 117     249 / 221
+//   with stage seeds         8.8 / 5.6  17.8 / 15.9  33.2 / 38.5  39.4 / 46.2
+//     FP16                 15.5 / 11.5  27.9 / 26.9  46.6 / 54.5  58.6 / 66.2
+//     D3Q27                 12.8 / 7.0  24.7 / 19.6  49.5 / 47.7  57.0 / 58.8
+//     D3Q27 FP16           19.5 / 12.3  36.8 / 30.1  66.3 / 62.5  77.8 / 74.1  96.9 / 93.8   179 / 178
+// The direct loads of a run cost a 16-bit forward step less than the staged
+// ring does at every size measured; 4 194 304 cells is the largest of them.
 bool marches(const lbm_handle& h, bool adjoint, bool stage) {
     const bool wide = (adjoint ? h.lam_storage : h.storage) == LBM_STORE_F32, q27 = h.Q == 27;
     int64_t most;
@@ -1489,7 +1493,7 @@ void check_errflag(lbm_handle& h) {
     if (e) {
         CK(cudaMemsetAsync(h.errflag.p, 0, sizeof(int), h.stream));
         // blocks that gave up did not take their ticket of a sum
-        CK(cudaMemsetAsync(h.counter.p, 0, 2 * sizeof(unsigned), h.stream));
+        CK(cudaMemsetAsync(h.counter.p, 0, sizeof(unsigned), h.stream));
         throw CudaError("a staged bulk copy or a barrier between steps did not complete within its bounded wait");
     }
 }
@@ -1630,12 +1634,9 @@ DesignArgs design_args(lbm_handle& h) {
 }
 
 // ------------------------------------------------------------ host arrays
-// A call's FP64 results pass through pinned FP32 staging in pieces of at most
-// PIN_CAP bytes: the copy runs at the link's rate and the conversion, which
-// first touches the pages of the caller's new array, on several threads (one
-// thread took 5 ms for 4.2M cells; an FP64 copy into untouched pages 7.6 ms).
-// in (host FP64) -> dev (FP32), narrowed on the device in pieces of at most
-// IO_CAP bytes; with `unit` a value outside [0, 1] sets the handle's flag.
+// A call's FP64 inputs are copied as they are and narrowed on the device, in
+// pieces of at most IO_CAP bytes; with `unit` a value outside [0, 1] sets the
+// handle's flag.
 constexpr int64_t IO_CAP = 64 << 20;
 
 // (from the list: a new handle's first call allocates nothing)
@@ -1643,10 +1644,9 @@ void io_buffer(lbm_handle& h, DevBuf& io, int64_t values) {
     io.alloc_pooled((size_t)std::min<int64_t>(values * 8, IO_CAP), &h.device_bytes, h.device, h.stream);
 }
 
-//
-// Up to HOST_VALUES values the host converts and checks: fewer calls than the
-// list, the kernel and the flag take (set_design of 1280 cells 50 -> 33 us).
-// Returns false for a value outside [0, 1] seen there.
+// in (host FP64) -> dev (FP32).  Up to HOST_VALUES values the host converts and
+// checks: fewer calls than the list, the kernel and the flag take (set_design of
+// 1280 cells 50 -> 33 us).  Returns false for a value outside [0, 1] seen there.
 constexpr int64_t HOST_VALUES = 16 << 10;
 
 bool upload(lbm_handle& h, const double* in, float* dev, int64_t n, bool unit) {
@@ -1681,7 +1681,11 @@ bool take_flag(lbm_handle& h) {
     return bad != 0;
 }
 
-// dev (FP32) -> out (host FP64); returns whether every value is finite.
+// dev (FP32) -> out (host FP64); returns whether every value is finite.  The
+// values pass through pinned FP32 staging in pieces of at most PIN_CAP bytes: the
+// copy runs at the link's rate and the conversion, which first touches the pages
+// of the caller's new array, on several threads (one thread took 5 ms for 4.2M
+// cells; an FP64 copy into untouched pages 7.6 ms).
 bool download(lbm_handle& h, const PinLease& pin, const float* dev, double* out, int64_t n) {
     float* st = pin.floats();
     const int64_t piece = PIN_CAP / 4;

@@ -474,9 +474,9 @@ LBM_API lbm_status lbm_slab_gradient(lbm_handle* h, double* grad, size_t n);
 /* No counterpart in the reference.  For callers that cannot allocate device
  * memory -- code inside another framework's memory pool or arena (the pool
  * owns all device memory), embedded hosts that fix their device budget up
- * front -- and that already hold a state on the device: the admission statistics of that one
- * state, computed by the same compensated reduction the stepping kernels run
- * every step (LbmProblem::admit quantities, solver.rs:714-755).
+ * front -- and that already hold a state on the device: the admission
+ * statistics of that one state, its sums compensated as the stepping kernels'
+ * are (LbmProblem::admit quantities, solver.rs:714-755).
  *
  *   populations  device, FP32, plane-major f[q*cells + cell] (unshifted f),
  *                velocity order of the lattice as in lbm_get_populations.
