@@ -75,7 +75,7 @@ __device__ __forceinline__ void adj_one_cell(const AdjArgs& a, const S* st, int 
     float om = a.P.omega, omm = a.P.om;
     if (a.omega_cell) om = omm = a.omega_cell[x];  // Tau::PerCell (BGK only)
     const bool post = (STG && a.stage) || (a.port_transpose && (m & MASK_PORT));
-    float ab = collide_vjp<Q, COLL, sizeof(T) == 2>(v, rp, u, st->alpha[c], a.P, om, omm, post ? 1.f : k_out) *
+    float ab = collide_vjp<Q, COLL, keeps_order<T>>(v, rp, u, st->alpha[c], a.P, om, omm, post ? 1.f : k_out) *
                a.in_scale_inv;
     if constexpr (STG) {
         if (a.stage) {
@@ -84,7 +84,7 @@ __device__ __forceinline__ void adj_one_cell(const AdjArgs& a, const S* st, int 
 #pragma unroll
             for (int e = 0; e < 6; ++e) Sm[e] = st->rec[4 + e][a.recd[4 + e] + c];
             const PortMap* pm = (m & MASK_PORT) ? &a.ports[((m >> MASK_PORT_SHIFT) & 7u) - 1] : nullptr;
-            ab += response_vjp<Q, sizeof(T) == 2>(rp, u, Sm, st->alpha[c], pm ? pm->dp_weight : 0.f, pm != nullptr,
+            ab += response_vjp<Q, keeps_order<T>>(rp, u, Sm, st->alpha[c], pm ? pm->dp_weight : 0.f, pm != nullptr,
                                                   a.seed, a.P, fb);
 #pragma unroll
             for (int q = 0; q < Q; ++q) v[q] = fmaf(fb[q], s_in, v[q]);
@@ -125,10 +125,10 @@ __device__ __forceinline__ void adj_one_cell(const AdjArgs& a, const S* st, int 
 // is bound by latency and instruction issue, not bytes, and a third block's
 // warps hide more of it (us per step with two / three, FP16: 256x128x128 126.3 /
 // 109.4, 128^3 69.7 / 57.2, D3Q27 192x128x128 128.4 / 113.9, with the registers
-// spilled).  The seeded D3Q27 step spills too much for it (250 / 258), and FP32
-// storage keeps two (135.1 / 135.9, 71.6 / 72.4).
+// spilled).  The seeded D3Q27 step of FP16 spills too much for it (250 / 258),
+// and FP32 storage keeps two (135.1 / 135.9, 71.6 / 72.4).
 template <int Q, int COLL, typename T, int AL, int STG>
-__global__ void __launch_bounds__(TPB, (sizeof(T) == 2 && !(STG && Q == 27) ? 3 : 2)) k_adjoint(AdjArgs a) {
+__global__ void __launch_bounds__(TPB, (sizeof(T) == 2 && !(STG && Q == 27 && keeps_order<T>) ? 3 : 2)) k_adjoint(AdjArgs a) {
     constexpr int NREC = STG ? 10 : 4;
     using S = AdjStage<Q, T, NREC>;
     constexpr int NCOPY = Q + NREC + 2;  // runs of lambda, the record, mask and alpha
@@ -188,11 +188,11 @@ __global__ void __launch_bounds__(TPB, (sizeof(T) == 2 && !(STG && Q == 27) ? 3 
         const float k_out = a.out_scale * a.in_scale_inv;  // stored input -> stored output
         using Z = ZWall<Q>;
         // FP16 256x128x128: 114.0 -> 109.4 us per step, D3Q27 192x128x128 148 -> 114,
-        // with stage seeds 277 -> 250; the seeded D3Q19 step at three blocks per SM
-        // has no registers to spare (263 -> 267).  FP32 storage is bound by bandwidth
+        // with stage seeds 277 -> 250; the seeded D3Q19 step of FP16 at three blocks
+        // per SM has no registers to spare (263 -> 267).  FP32 storage is bound by bandwidth
         // and gains nothing (D3Q27 lost 10% to the registers), nor does the forward
         // step, whose registers then spill (124 -> 135 us).
-        constexpr bool PREFETCH = sizeof(T) == 2 && !(STG && Q == 19);
+        constexpr bool PREFETCH = sizeof(T) == 2 && !(STG && Q == 19 && keeps_order<T>);
         ZWalk z(a.G, blockIdx.x * TILE + c0, gridDim.x * TILE);
         for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, z.next()) {
             const uint32_t x = tile * TILE + c0;

@@ -986,12 +986,12 @@ __device__ __forceinline__ Macro collide_fused_dp(float (&vf)[Q], float alpha_f,
 // multiples of the precomputed moments of their basis vectors.  Then the
 // Brinkman chain F = rho (a - alpha u), u = (m/rho + a/2)/(1 + alpha/2).
 //
-// HALF: the cotangent is stored in 16 bits.  Its values round every step, so
+// HALF: the cotangent is stored in FP16.  Its values round every step, so
 // another order of these operations gives another trajectory, off by the
 // storage's noise: like the 16-bit forward step (collide_fused) this one keeps
 // its order, the moments of gb itself and the cotangents of eq, src and the
-// Brinkman chain in turn.  (The collected form would take 101 us of an FP16 step
-// of 256x128x128 cells where this one takes 110.)
+// Brinkman chain in turn.  (The collected form would take 101 us of a step of
+// 256x128x128 cells where this one takes 110.)
 template <int Q, int COLL, bool HALF>
 __device__ __forceinline__ float collide_vjp(float (&gb)[Q], float rp, const float (&u)[3], float alpha,
                                              const Physics& P, float om, float omm, float k = 1.f) {
@@ -1303,9 +1303,9 @@ __device__ __forceinline__ void second_moments(const float (&g)[Q], float (&S)[6
 // the Brinkman velocity u and the second moments S of g.  fb = d/dg; returns
 // the cotangent of alpha.  The responses depend on g only through these
 // moments, so the adjoint step can seed a state from its record alone.
-// HALF: the seed enters a cotangent stored in 16 bits, whose trajectories keep
+// HALF: the seed enters a cotangent stored in FP16, whose trajectories keep
 // their order of operations (collide_vjp), a dozen divisions per cell and all
-// (263 us per seeded FP16 step of 256x128x128 cells, 161 without them).
+// (263 us per seeded step of 256x128x128 cells, 161 without them).
 template <int Q, bool HALF>
 __device__ __forceinline__ float response_vjp(float rp, const float (&u)[3], const float (&S)[6], float alpha,
                                               float dpw, bool port, const SeedParams& sp, const Physics& P,
@@ -1679,6 +1679,10 @@ __device__ void finish_sums(Sums<NS> v, double* out, const Reduce& red) {
 #define LBM_PASTE_(a, b) a##_##b
 #define LBM_PASTE(a, b) LBM_PASTE_(a, b)
 #define LBM_PART_NAME(name) LBM_PASTE(name, LBM_PART)
+
+// Whether cotangents stored as T keep the order of operations of FP16 (HALF).
+template <typename T>
+constexpr bool keeps_order = std::is_same<T, __half>::value;
 
 #define LBM_STORAGE_DISPATCH(storage, T, ...)            \
     switch (storage) {                                   \

@@ -286,14 +286,14 @@ __global__ void __launch_bounds__(MT, MB) k_march_adjoint(const __grid_constant_
             float om = a.P.omega, omm = a.P.om;
             if (a.omega_cell) om = omm = a.omega_cell[x];
             const bool post = stage_on || (m & MASK_PORT);
-            float ab = collide_vjp<Q, COLL, sizeof(T) == 2>(v, rp, u, alpha, a.P, om, omm, post ? 1.f : k_out) * in_inv;
+            float ab = collide_vjp<Q, COLL, keeps_order<T>>(v, rp, u, alpha, a.P, om, omm, post ? 1.f : k_out) * in_inv;
             const PortMap* pm = (m & MASK_PORT) ? &ports[((m >> MASK_PORT_SHIFT) & 7u) - 1] : nullptr;
             if constexpr (STG) {
                 if (stage_on) {
                     float Sm[6], fb[Q];
 #pragma unroll
                     for (int e = 0; e < 6; ++e) Sm[e] = rec[(size_t)(4 + e) * n + x];
-                    ab += response_vjp<Q, sizeof(T) == 2>(rp, u, Sm, alpha, pm ? pm->dp_weight : 0.f, pm != nullptr,
+                    ab += response_vjp<Q, keeps_order<T>>(rp, u, Sm, alpha, pm ? pm->dp_weight : 0.f, pm != nullptr,
                                                           a.seed, a.P, fb);
 #pragma unroll
                     for (int q = 0; q < Q; ++q) v[q] = fmaf(fb[q], s_in, v[q]);

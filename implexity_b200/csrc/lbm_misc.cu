@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(BLOCK) k_objective(ObjArgs a) {
         const float* u = M.u;
         {
             float fb[Q];
-            const float abar = response_vjp<Q, sizeof(TL) == 2>(M.rp, M.u, S, alpha, pm ? pm->dp_weight : 0.f,
+            const float abar = response_vjp<Q, keeps_order<TL>>(M.rp, M.u, S, alpha, pm ? pm->dp_weight : 0.f,
                                                                 pm != nullptr, sp, a.P, fb);
             a.abar_final[x] = abar;
             a.phibar[x] = (float)a.w[5];

@@ -1870,19 +1870,20 @@ SeedParams stage_seed(const lbm_handle& h, const double* w, double scale) {
     return sp;
 }
 
-// The scales of a stored FP32 cotangent are powers of two: their quotients are
+// The scales of a stored FP32 or BF16 cotangent are powers of two: their quotients are
 // exact, where a rounded one (1 +- 6e-8) enters every step of a segment alike
 // and made the whole horizon gradient too long by up to 3e-6 after 400 steps.
-// A 16-bit cotangent is scaled to a root mean square of one: nearly uniform
+// An FP16 cotangent is scaled to a root mean square of one: nearly uniform
 // values then lie where the spacing of the format halves.  The nearest power of
-// two would put them anywhere between 0.7 and 1.4 (FP16 gradients of D3Q19 MRT
-// and D3Q27 horizons: 3.4e-4 and 2.0e-4 off FP64 instead of 1.3e-4 and 1.5e-4).
+// two would put them anywhere between 0.7 and 1.4 (gradients of D3Q19 MRT and
+// D3Q27 horizons: 3.4e-4 and 2.0e-4 off FP64 instead of 1.3e-4 and 1.5e-4; of BF16
+// they are the closer ones with a power of two, 1.1e-3 and 1.4e-3 for 2.4e-3).
 float power_of_two(double v) {
     if (!(v > 0) || !std::isfinite(v)) return 1.f;
     const double p = std::exp2(std::round(std::log2(v)));
     return p >= 1e-37 && p <= 1e37 ? (float)p : 1.f;
 }
-bool exact_scales(const lbm_handle& h) { return h.lam_storage == LBM_STORE_F32; }
+bool exact_scales(const lbm_handle& h) { return h.lam_storage != LBM_STORE_F16; }
 
 double seed(lbm_handle& h, const double* w, AdjState& st, float* record, double stage_scale = 1.0) {
     int64_t* ctr = &h.device_bytes;
