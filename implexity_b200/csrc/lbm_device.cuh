@@ -1109,7 +1109,7 @@ __device__ __forceinline__ float collide_vjp(float (&gb)[Q], float rp, const flo
         mul(H2, F, H2F);
         const float usq = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
         rho_bar = Z0 * (1.f - 1.5f * usq) + 3.f * (u[0] * Z1[0] + u[1] * Z1[1] + u[2] * Z1[2]) +
-                        4.5f * (u[0] * Z2u[0] + u[1] * Z2u[1] + u[2] * Z2u[2]);
+                  4.5f * (u[0] * Z2u[0] + u[1] * Z2u[1] + u[2] * Z2u[2]);
         float ub[3], Fb[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {

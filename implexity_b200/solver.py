@@ -257,7 +257,15 @@ class LbmSolver:
         "final") or of their mean over the horizon's states ("time_average",
         horizon mode, problems with solver_options.time_average).  Horizon
         checkpointing is a state every `checkpoint_every` steps ("every") or
-        the binomial schedule over `snapshots` states ("binomial")."""
+        the binomial schedule over `snapshots` states ("binomial").
+
+        Device memory of the horizon mode: with checkpoint_every=0 and no
+        record_budget_bytes, the records of the whole trajectory (16 bytes
+        per cell and state, 40 for the time average) where they take at most
+        16 GiB and half of the free memory; else, and with an interval K given,
+        steps / K states and K records; with "binomial", `snapshots` states
+        and one record.  Up to 16 GiB of it stays with the library for the next
+        gradient and goes back with the last open solver."""
         w = np.zeros(_abi.N_RESPONSES)
         w[: len(weights)] = np.asarray(weights, dtype=float)
         o = _abi.AdjointOpts()

@@ -255,7 +255,7 @@ typedef struct {
     int32_t mode;             /* lbm_adjoint_mode */
     int32_t lambda_storage;   /* lbm_storage of the adjoint populations */
     int64_t checkpoint_every; /* HORIZON: K (<= 0: every record of the trajectory is kept where they fit in
-                                 16 GB and half of the free memory, else K = sqrt(step_count)) */
+                                 16 GiB and half of the free memory, else K = sqrt(step_count)) */
     int64_t max_iterations;   /* STEADY: cap */
     int64_t check_every;      /* STEADY: residual readback period */
     double tolerance;         /* STEADY: relative residual */
