@@ -1333,7 +1333,7 @@ void inspect(lbm_handle& h, StepDiag* diag, float* record, bool record_s = false
 //   with stage seeds         8.8 / 5.6  17.8 / 15.9  33.2 / 38.5  39.4 / 46.2
 //     FP16                 15.5 / 11.5  27.9 / 26.9  46.6 / 54.5  58.6 / 66.2
 //     D3Q27                 12.8 / 7.0  24.7 / 19.6  49.5 / 47.7  57.0 / 58.8
-//     D3Q27 FP16           19.5 / 12.3  36.8 / 30.1  66.3 / 62.5  77.8 / 74.1  96.9 / 93.8   179 / 178
+//     D3Q27 FP16           19.5 / 12.3  36.8 / 30.1  62.5 / 62.5  74.9 / 74.1  93.2 / 93.8   172 / 178
 // The direct loads of a run cost a 16-bit forward step less than the staged
 // ring does at every size measured; 4 194 304 cells is the largest of them.
 bool marches(const lbm_handle& h, bool adjoint, bool stage) {
