@@ -357,8 +357,9 @@ BlockList& block_list() {
 }
 
 void destroy_block(const Block& b) {
+    cudaEventSynchronize(b.last_use);
     cudaEventDestroy(b.last_use);
-    cudaFree(b.p);  // (waits for the device: a last use may be in flight)
+    cudaFree(b.p);
 }
 // Frees a device's oldest idle blocks until `keep` bytes are left.
 void shrink_idle(BlockList& L, int device, size_t keep) {
