@@ -533,13 +533,19 @@ struct DevBuf {
 // not page-lock memory again (10 to 50 ms for 16 MB on a shared host).  The
 // list keeps at most four buffers (PIN_CAP bytes each at most) while handles
 // exist and is emptied with the last one; a lease belongs to one call, so
-// threads with handles of their own do not meet in a buffer.
+// threads with handles of their own do not meet in a buffer.  Up to PIN_SMALL
+// bytes plain memory does as well: locking 64 KB takes 1 to 3 ms here, a copy
+// through the driver's own staging 1 us more.  So the list locks a small buffer
+// only for the lease after PIN_SMALL_USES of them: a program that opens a small
+// problem once never pays for it.
 constexpr int64_t PIN_CAP = 32 << 20;
+constexpr size_t PIN_SMALL = 64 << 10;
+constexpr int64_t PIN_SMALL_USES = 1000;
 
 struct PinList {
     std::mutex mu;
     std::vector<std::pair<void*, size_t>> idle;  // never grows past its reserve: a lease ends without allocating
-    int64_t handles = 0;
+    int64_t handles = 0, small_uses = 0;
     PinList() { idle.reserve(8); }
 };
 PinList& pin_list() {
@@ -553,16 +559,18 @@ void pin_handles(int by) {
     if (L.handles > 0) return;
     for (auto& b : L.idle) cudaFreeHost(b.first);
     L.idle.clear();
+    L.small_uses = 0;
 }
 
 struct PinLease {
     void* p = nullptr;
     size_t bytes = 0;
-    bool pinned = true;  // false: the host would not lock more pages; the copies then go through the driver's
+    bool pinned = true;  // false: plain memory; the copies go through the driver's own staging
     explicit PinLease(size_t want) {
-        size_t size = 64 << 10;
+        size_t size = PIN_SMALL;
         while (size < want) size *= 2;
         PinList& L = pin_list();
+        bool lock_pages = true;
         {
             std::lock_guard<std::mutex> lock(L.mu);
             for (size_t i = 0; i < L.idle.size(); ++i)
@@ -572,8 +580,9 @@ struct PinLease {
                     L.idle.erase(L.idle.begin() + (std::ptrdiff_t)i);
                     return;
                 }
+            lock_pages = size > PIN_SMALL || ++L.small_uses > PIN_SMALL_USES;
         }
-        if (cudaMallocHost(&p, size) != cudaSuccess) {
+        if (!lock_pages || cudaMallocHost(&p, size) != cudaSuccess) {  // (or the host would not lock more)
             cudaGetLastError();
             p = std::malloc(size);
             if (!p) throw std::bad_alloc();
